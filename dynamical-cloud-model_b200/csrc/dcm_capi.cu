@@ -95,6 +95,7 @@ struct dcm_handle {
     // captured pressure solves (FP64 and mixed), rebuilt when their
     // arguments change
     SolveGraph g64, g32;
+    DirectPlan direct;  // direct corrections of the mixed solve
     // solver loops: 1 graph-driven, 2 graph-driven without programmatic
     // dependent launch, 0 host-polled
     int graphs = 1;
@@ -386,6 +387,7 @@ extern "C" int dcm_create(const dcm_grid* g, int device, dcm_handle** out) {
     CK(cudaStreamCreateWithFlags(&h->st, cudaStreamNonBlocking));
     solver_init();
     mpdata_init();
+    direct_init();
     CK(cudaEventCreate(&h->ev0));
     CK(cudaEventCreate(&h->ev1));
     const size_t I2 = g->ip + 2, J2 = g->jp + 2, K2 = g->kp + 2;
@@ -477,6 +479,8 @@ extern "C" int dcm_create(const dcm_grid* g, int device, dcm_handle** out) {
     CK(cudaMalloc(&h->S2, sizeof(SolverScalars)));
     CK(cudaMemset(h->S2, 0, sizeof(SolverScalars)));
     CK(cudaMallocHost(&h->hS2, sizeof(SolverScalars)));
+    if (direct_plan_build(d, ae, aw, an, as, au, ad, &h->direct) != DCM_OK)
+        return cuda_fail(h, cudaGetLastError(), "direct solver tables");
     CK(cudaStreamSynchronize(h->st));
     *out = h;
     return DCM_OK;
@@ -501,6 +505,7 @@ extern "C" int dcm_destroy(dcm_handle* h) {
     for (double* p : h->slots) free_field(p);
     for (float* p : h->fslots) free_field(p);
     cudaFree(h->metric_block_f);
+    cudaFree(h->direct.block);
     cudaFree(h->sg_lamsq);
     cudaFree(h->dense_stage);
     cudaFree(h->S2);
@@ -1022,6 +1027,7 @@ SolverWork<float> solver_work_f(dcm_handle* h) {
     w.cheb = h->cfg.precond == 1 ? 1 : 0;
     w.cheb_lo = h->cfg.precond_lo > 0.0 ? h->cfg.precond_lo : 0.05;
     w.round_budget = h->round_budget;
+    w.direct = &h->direct;
     return w;
 }
 

@@ -31,6 +31,47 @@ struct SolverScalars {
     int restarts;  // restarts of this solve
     int cycle_it;  // FP32 iterations since the last FP64 update
     double crnorm;  // (cr, cr) of the shadow residual
+    int direct;     // mixed form: another direct correction follows (k_direct.cu)
+    int dir_runs;   // direct corrections of this solve
+};
+
+// per-axis coefficients of the 7-point operator (set_mat_a)
+template <typename T>
+struct Coef {
+    const T *ae, *aw;  // per i
+    const T *an, *as;  // per j
+    const T *au, *ad;  // per k
+};
+
+// ---- direct corrections of the mixed form's solve (k_direct.cu) -------------
+// The domains that take them, by interior points.  Measured per step (mixed
+// form, precond 1, iterations -> corrections): 97x75x61 7.4 -> 0.4 ms,
+// 256x256x128 34 -> 2.6 ms.  Smaller domains would gain too, but keep the
+// FP32 iterations: a step of 81x45x32 takes 4 ms, and the iteration counts
+// that dcm_step reports there are what the sweeps and launch shapes are
+// compared by.  Larger ones keep them because of p's additive constant, which
+// no velocity depends on: there the iterations' round-off and restarts move
+// it (2 of 21 seeded 384x256x256 convections: a mean of 4 % of p's spread,
+// and far above it), so a corrected solve would return another p.  Up to
+// 2e7 points it stayed below 1e-6 (120 solves).
+constexpr long long DIRECT_MIN_POINTS = 1 << 17;
+constexpr long long DIRECT_MAX_POINTS = 1 << 24;
+// a correction is followed by another while it lowers the residual by this
+// factor (one lowers it by about 1e-4); else the iterations take over
+constexpr double DIRECT_CONTRACTION = 0.25;
+constexpr int DIRECT_MAX_RADICES = 12;
+constexpr size_t DIRECT_MAX_SMEM = 227 * 1024;  // of one transform block
+
+struct AxisPlan {
+    int n = 0, nrad = 0, rad[DIRECT_MAX_RADICES] = {0};
+    const float2* tw = nullptr;  // n roots of unity
+    const float* lam = nullptr;  // n eigenvalues of the axis' circulant
+};
+struct DirectPlan {
+    bool ok = false;
+    AxisPlan axis[2];  // x, y
+    const double *w = nullptr, *g = nullptr, *l = nullptr;  // mean mode (k_zsolve)
+    void* block = nullptr;  // the device tables
 };
 
 // One pressure solve captured as a CUDA graph: the iteration loop is a
@@ -40,7 +81,7 @@ struct SolverScalars {
 struct SolveGraph {
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
-    cudaStream_t side[2] = {nullptr, nullptr};  // capture streams of the loop bodies
+    cudaStream_t side[3] = {nullptr, nullptr, nullptr};  // capture streams of the loop bodies
     // key: everything the captured launches depend on
     const void* key_ptr[6] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
     double key_d[3] = {0, 0, 0};
@@ -111,7 +152,26 @@ struct SolverWork {
     // FP64: domains of at most this many interior points solve in one
     // thread-block cluster (k_bicgstab_small); 0 = never
     long long small_max = 0;
+    // mixed form: direct corrections ahead of the iterations (null or !ok: none)
+    const DirectPlan* direct = nullptr;
 };
+
+// direct corrections (k_direct.cu)
+void direct_init();
+// tables for the grid's operator, or ok = false where the rule excludes it
+int direct_plan_build(const Dims& d, const std::vector<double>& ae, const std::vector<double>& aw,
+                      const std::vector<double>& an, const std::vector<double>& as,
+                      const std::vector<double>& au, const std::vector<double>& ad,
+                      DirectPlan* plan);
+// x += A^-1 r (r FP32, x FP64; work: one FP32 field)
+void direct_correction(const DirectPlan& P, const Dims& d, const Coef<float>& c, const float* r,
+                       float* work, double* x, cudaStream_t st);
+// r = b - A x and the loop's decision into S->direct, S->done, S->status (and
+// the WHILE node's condition)
+void direct_residual(const Dims& d, const Coef<double>& c, const double* x, const double* b,
+                     float* r, double tol, int itmax, int max_rounds, bool first, const Red2& red,
+                     int max_blocks, SolverScalars* S, const cudaGraphConditionalHandle* cond,
+                     cudaStream_t st);
 
 // one-time setup of the solver kernels (shared-memory limits, the probe of
 // programmatic launches in graphs); called at handle creation, outside any

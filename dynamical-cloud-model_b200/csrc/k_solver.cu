@@ -61,13 +61,6 @@ __device__ __forceinline__ void pdl_launch() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
-template <typename T>
-struct Coef {
-    const T *ae, *aw;  // per i
-    const T *an, *as;  // per j
-    const T *au, *ad;  // per k
-};
-
 struct SolverArgs {
     Dims d;
     int itmax;
@@ -95,6 +88,9 @@ struct SolverArgs {
     int cond_max = 0;
     // launch with programmatic stream serialisation (pdl_wait)
     int pdl = 0;
+    // mixed form: the iterations follow direct corrections, whose counts and
+    // rounds they continue
+    int after_direct = 0;
     // |omega| below this ends an FP64 solve with DCM_E_BREAKDOWN; the
     // reference's tiny is the default-real literal 1.e-16 (dynamics.f90:321)
     double tiny = (double)1.e-16f;
@@ -1354,6 +1350,12 @@ __global__ void k_outer_cond(cudaGraphConditionalHandle h, const SolverScalars* 
     cudaGraphSetConditional(h, S->done ? 0u : 1u);
 }
 
+// Mixed form: the FP32 iterations follow where the direct corrections did not
+// end the solve.
+__global__ void k_branch_iterate(cudaGraphConditionalHandle h, const SolverScalars* S) {
+    cudaGraphSetConditional(h, S->done ? 0u : 1u);
+}
+
 // Condition of the IF node of the mixed solve: the FP32 iterations paused
 // for a reliable update (otherwise they finished).
 __global__ void k_branch_pause(cudaGraphConditionalHandle h, SolverScalars* S) {
@@ -2061,14 +2063,16 @@ __global__ void __launch_bounds__(256) k_ru_residual(SolverArgs a, Coef<double> 
             double sc = sqrt(s[0]);
             sc = sc > 0.01 ? sc : 0.01;  // dynamics.f90:370-371
             S->sc_err = sc;
-            S->it = 0;
             S->status = 0;
-            S->updates = 0;
-            S->rounds = 0;
             S->cycles = 0;
             S->ru_runs = 0;
             S->restarts = 0;
-            S->fresh = 0;
+            S->fresh = a.after_direct;  // p = v1 = 0 whatever the count says
+            if (!a.after_direct) {
+                S->it = 0;
+                S->updates = 0;
+                S->rounds = 0;
+            }
         }
         const double err = sqrt(s[1]) / S->sc_err;
         S->err = err;
@@ -2173,9 +2177,20 @@ int refine_run(SolverWork<float>& wf, SolverWork<double>& wd, const Dims& d, dou
     static const int gfull = persistent_grid(k_ru_residual<false>);
     const int g = red_grid(a, gfull, a.nkt, a.ni);
     const dim3 gi = interior_grid(d, d.kp), bl(BX, BY);
+    const bool direct = wf.direct && wf.direct->ok;
+    a.after_direct = direct ? 1 : 0;
+    const int max_rounds = wf.round_budget > 0 ? wf.round_budget : itmax + max_updates + 1;
+    auto start = [&](cudaStream_t s) { k_ru_begin<<<1, 1, 0, s>>>(wf.S, delta); };
+    // the residual of a direct phase; the correction it calls for
+    auto dir_residual = [&](cudaStream_t s, bool first, const cudaGraphConditionalHandle* h) {
+        direct_residual(d, cd, x, b, wf.r, tol, itmax, max_rounds, first, wd.red, wf.max_blocks,
+                        wf.S, h, s);
+    };
+    auto dir_correct = [&](cudaStream_t s) {
+        direct_correction(*wf.direct, d, cf, wf.r, wf.sA, x, s);
+    };
     auto begin = [&](cudaStream_t s) {
         cudaMemsetAsync(dx, 0, d.n() * sizeof(float), s);
-        k_ru_begin<<<1, 1, 0, s>>>(wf.S, delta);
         ProfScope ps(P_SETUP, s);
         k_ru_residual<true><<<g, bl, 0, s>>>(a, cd, cf, x, b, wf.r, wf.rh, wf.cr, wd.red, wf.S);
     };
@@ -2187,18 +2202,18 @@ int refine_run(SolverWork<float>& wf, SolverWork<double>& wd, const Dims& d, dou
         ProfScope ps(P_SETUP, s);
         k_ru_residual<false><<<g, bl, 0, s>>>(a, cd, cf, x, b, wf.r, wf.rh, wf.cr, wd.red, wf.S);
     };
+    auto last_add = [&](cudaStream_t s) {
+        // the correction accumulated since the last update (zero after one)
+        ProfScope ps(P_UPDATE, s);
+        k_ru_add<<<gi, bl, 0, s>>>(d, x, dx, wf.S);
+    };
     auto finish = [&](cudaStream_t s) {
-        {
-            // the correction accumulated since the last update (zero after one)
-            ProfScope ps(P_UPDATE, s);
-            k_ru_add<<<gi, bl, 0, s>>>(d, x, dx, wf.S);
-        }
         k_ru_end<<<1, 1, 0, s>>>(wf.S, wd.S);
         ProfScope ps(P_POST, s);
         k_bicg_post<double, float><<<gi, bl, 0, s>>>(d, x, sw, dzn, wd.S, 1);
     };
-    const int max_rounds = wf.round_budget > 0 ? wf.round_budget : itmax + max_updates + 1;
-    // the whole mixed solve into the graph being captured on `s0`:
+    // the iterations into the graph being captured on `s0`, their loop bodies
+    // on the side streams lvl and lvl + 1:
     //   WHILE (not done) {                           one FP64 update cycle
     //       WHILE (not done, not paused) { FP32 iteration }
     //       IF (paused) { reliable update }
@@ -2207,16 +2222,14 @@ int refine_run(SolverWork<float>& wf, SolverWork<double>& wd, const Dims& d, dou
     // an iteration is its five (or nine) kernels and nothing else.  Both
     // loops are bounded: a cycle starts with pause = 0, so every cycle that
     // does not end the solve counts an iteration against max_rounds.
-    auto emit = [&](cudaStream_t s0, SolveGraph& G) {
-        if (!side_streams(G)) return false;
-        CaptureGuard cgd;
+    auto emit_iterations = [&](cudaStream_t s0, SolveGraph& G, int lvl) {
         cudaGraphConditionalHandle ho{};
         cudaGraph_t body[1] = {nullptr};
         begin(s0);
         bool good = capture_cond_handle(s0, &ho, 0);
         if (good) k_outer_cond<<<1, 1, 0, s0>>>(ho, wf.S);
         good = good && capture_cond_node(s0, ho, cudaGraphCondTypeWhile, 1, body);
-        good = good && capture_into(G.side[0], body[0], [&](cudaStream_t s) {
+        good = good && capture_into(G.side[lvl], body[0], [&](cudaStream_t s) {
                    cudaGraphConditionalHandle hi{}, hb{};
                    cudaGraph_t in[1] = {nullptr}, br[1] = {nullptr};
                    SolverArgs ai = af;
@@ -2226,17 +2239,48 @@ int refine_run(SolverWork<float>& wf, SolverWork<double>& wd, const Dims& d, dou
                    ai.cond = hi;
                    ai.cond_max = max_rounds;
                    ai.pdl = g_pdl_graphs && wf.pdl;
-                   g2 = g2 && capture_into(G.side[1], in[0], [&](cudaStream_t s2) {
+                   g2 = g2 && capture_into(G.side[lvl + 1], in[0], [&](cudaStream_t s2) {
                             for (int n = 0; n < ITERS_PER_BODY; n++)
                                 launch_iteration<float>(ai, cf, wf, dx, s2);
                         });
                    g2 = g2 && capture_cond_handle(s, &hb, 0);
                    if (g2) k_branch_pause<<<1, 1, 0, s>>>(hb, wf.S);
                    g2 = g2 && capture_cond_node(s, hb, cudaGraphCondTypeIf, 1, br);
-                   g2 = g2 && capture_into(G.side[1], br[0], update);
+                   g2 = g2 && capture_into(G.side[lvl + 1], br[0], update);
                    k_outer_cond<<<1, 1, 0, s>>>(ho, wf.S);
                    if (!g2) good = false;
                });
+        last_add(s0);
+        return good;
+    };
+    // the whole mixed solve into the graph being captured on `s0`; with direct
+    // corrections
+    //   residual, WHILE (it calls for one) { correction, residual }
+    //   IF (not done) { the iterations }
+    auto emit = [&](cudaStream_t s0, SolveGraph& G) {
+        if (!side_streams(G)) return false;
+        CaptureGuard cgd;
+        bool good = true;
+        start(s0);
+        if (!direct) {
+            good = emit_iterations(s0, G, 0);
+        } else {
+            cudaGraphConditionalHandle hd{}, hk{};
+            cudaGraph_t body[1] = {nullptr}, rest[1] = {nullptr};
+            good = capture_cond_handle(s0, &hd, 0);
+            if (good) dir_residual(s0, true, &hd);
+            good = good && capture_cond_node(s0, hd, cudaGraphCondTypeWhile, 1, body);
+            good = good && capture_into(G.side[0], body[0], [&](cudaStream_t s) {
+                       dir_correct(s);
+                       dir_residual(s, false, &hd);
+                   });
+            good = good && capture_cond_handle(s0, &hk, 0);
+            if (good) k_branch_iterate<<<1, 1, 0, s0>>>(hk, wf.S);
+            good = good && capture_cond_node(s0, hk, cudaGraphCondTypeIf, 1, rest);
+            good = good && capture_into(G.side[0], rest[0], [&](cudaStream_t s) {
+                       if (!emit_iterations(s, G, 1)) good = false;
+                   });
+        }
         finish(s0);
         return good && cudaPeekAtLastError() == cudaSuccess;
     };
@@ -2247,7 +2291,8 @@ int refine_run(SolverWork<float>& wf, SolverWork<double>& wd, const Dims& d, dou
         const void* kp[6] = {x, b, sw, dzn, dx, wf.S};
         const double kd[3] = {tol, delta, af.cheb ? wf.cheb_lo : 0.0};
         const int shape = af.by + 16 * af.tasks + 256 * af.ni + 16384 * af.fuse +
-                          65536 * af.cheb + 131072 * (wf.pdl ? 1 : 0) + 262144 * af.vw;
+                          65536 * af.cheb + 131072 * (wf.pdl ? 1 : 0) + 262144 * af.vw +
+                          2097152 * (direct ? 1 : 0);
         const int ki[6] = {itmax, max_updates, 1 + 2 * max_rounds, 16 * shape,
                            d.ip * 4096 + d.jp, d.kp};
         if (!G.matches(kp, kd, ki)) {
@@ -2270,9 +2315,23 @@ int refine_run(SolverWork<float>& wf, SolverWork<double>& wd, const Dims& d, dou
         }
         if (!ok(cudaGraphLaunch(G.exec, st))) return DCM_E_CUDA;
     } else {
-        begin(st);
+        start(st);
+        bool iterate = true;
+        if (direct) {
+            dir_residual(st, true, nullptr);
+            for (;;) {
+                cudaMemcpyAsync(hS_in, wf.S, sizeof(SolverScalars), cudaMemcpyDeviceToHost, st);
+                if (cudaStreamSynchronize(st) != cudaSuccess) return DCM_E_CUDA;
+                if (!hS_in->direct) break;
+                dir_correct(st);
+                dir_residual(st, false, nullptr);
+                if (cudaGetLastError() != cudaSuccess) return DCM_E_CUDA;
+            }
+            iterate = !hS_in->done;
+        }
+        if (iterate) begin(st);
         int launched = 0;
-        for (int round = 0;; round++) {
+        for (int round = 0; iterate; round++) {
             cudaMemcpyAsync(hS_in, wf.S, sizeof(SolverScalars), cudaMemcpyDeviceToHost, st);
             if (cudaStreamSynchronize(st) != cudaSuccess) return DCM_E_CUDA;
             if (hS_in->done || round > max_rounds) break;
@@ -2285,6 +2344,7 @@ int refine_run(SolverWork<float>& wf, SolverWork<double>& wd, const Dims& d, dou
                 launch_iteration<float>(af, cf, wf, dx, st);
             if (cudaGetLastError() != cudaSuccess) return DCM_E_CUDA;
         }
+        if (iterate) last_add(st);
         finish(st);
     }
     cudaMemcpyAsync(hS_in, wf.S, sizeof(SolverScalars), cudaMemcpyDeviceToHost, st);
@@ -2293,14 +2353,23 @@ int refine_run(SolverWork<float>& wf, SolverWork<double>& wd, const Dims& d, dou
     int status = hS_out->status;
     if (status == DCM_OK && !hS_in->done) status = DCM_E_NOCONV;  // host loop ran out
     if (use_graph && g_prof) {
-        // iterations, reliable updates and cycles the graph ran
-        const long long itr = hS_in->rounds, u = hS_in->ru_runs, cyc = hS_in->cycles;
-        g_prof->add(P_SETUP, u + 1);
-        g_prof->add(P_JACOBI, (fused_ok<float>(af) ? 2 : 6) * itr);
-        g_prof->add(P_MATVEC, (fused_ok<float>(af) && af.fuse_mv ? 1 : 2) * itr);
-        g_prof->add(P_UPDATE, itr + u + 1);
+        // direct corrections, iterations, reliable updates and cycles the graph ran
+        const long long dc = hS_in->dir_runs, u = hS_in->ru_runs, cyc = hS_in->cycles;
+        const long long itr = hS_in->rounds - dc;
+        const bool iterated = !direct || cyc > 0;
+        if (direct) {
+            g_prof->add(P_SETUP, dc + 1);
+            g_prof->add(P_JACOBI, dc * (d.ip > 1 ? 5 : 3));
+        }
+        if (iterated) {
+            g_prof->add(P_SETUP, u + 1);
+            g_prof->add(P_JACOBI, (fused_ok<float>(af) ? 2 : 6) * itr);
+            g_prof->add(P_MATVEC, (fused_ok<float>(af) && af.fuse_mv ? 1 : 2) * itr);
+            g_prof->add(P_UPDATE, itr + u + 1);
+            g_prof->add(P_OTHER, 3 * cyc + 1);
+        }
         g_prof->add(P_POST, 1);
-        g_prof->add(P_OTHER, 3 * cyc + 3);
+        g_prof->add(P_OTHER, direct ? 3 : 2);
     }
     if (rs) {
         rs->outer = hS_in->updates;

@@ -231,7 +231,13 @@ typedef struct {
     int precision;          /* 0 = FP64 (the reference's VAR_TYPE=1);
                                1 = FP32 fields; FP32 BiCGSTAB iterations on
                                an FP64 pressure with FP64 reliable updates,
-                               converged to ptol on the FP64 residual      */
+                               converged to ptol on the FP64 residual.  With
+                               uniform dx, dxn and uniform dy, dyn (and 2^17
+                               to 2^24 points) the FP64 residual is first
+                               lowered by direct corrections, FP32 solves of
+                               A dx = r by transforms in x and y and
+                               tridiagonal systems in z; the iterations
+                               follow where one does not contract it       */
     double inner_tol;       /* precision 1: reliable-update factor: the FP32
                                recursion stops for an FP64 update of p and
                                of the true residual when its residual has
@@ -264,12 +270,15 @@ typedef struct {
 
 typedef struct {
     int steps;              /* steps taken in this call                   */
-    int iters_last;         /* BiCGSTAB iterations of the last step       */
+    int iters_last;         /* BiCGSTAB iterations of the last step; each
+                               direct correction of the mixed form (see
+                               precision) counts as one                   */
     long long iters_total;  /* summed over the call                       */
     double err_last;        /* final relative residual of the last solve  */
     double ms_total;        /* device time of the call (CUDA events)      */
-    int updates_last;       /* precision 1: FP64 reliable updates of the
-                               last solve (0 for FP64)                     */
+    int updates_last;       /* precision 1: FP64 updates of the last solve,
+                               reliable updates and direct corrections
+                               (0 for FP64)                                */
     int restarts_last;      /* precision 1: of those, restarts after a
                                breakdown of the FP32 recursion             */
 } dcm_step_stats;
@@ -343,8 +352,8 @@ int dcm_horizontal_means_noalloc(int ip, int jp, int kp, const double *u,
  * time (CUDA events recorded on the launching stream around every launch of
  * dcm_step while timing is enabled).  dcm_profile_enable resets both.
  * Classes:
- * 0 solver setup, 1 Jacobi sweeps, 2 matvecs, 3 x/r update, 4 solver post,
- * 5 means+divergence, 6 sources, 7 Poisson rhs, 8 adv_ref_state,
+ * 0 solver setup (residuals), 1 Jacobi sweeps (and the kernels of direct
+ * corrections), 2 matvecs, 3 x/r update, 4 solver post, 5 means+divergence, 6 sources, 7 Poisson rhs, 8 adv_ref_state,
  * 9 MPDATA shift, 10 donor cell, 11 antidiffusive velocities, 12 beta,
  * 13 limiter, 14 MPDATA restore, 15 momentum, 16 other. */
 #define DCM_PROF_NCAT 17

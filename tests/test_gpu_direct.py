@@ -1,0 +1,103 @@
+"""GPU checks of the mixed form's direct corrections (Hartley transforms along
+x and y, tridiagonal systems along z, in FP32, on the FP64 residual).
+
+A step of domains above the size where they start, at transform lengths of
+every kind (powers of two, products of the other small radices, primes, a
+length whose tiles are narrower, 1), columns of one to sixteen levels per
+lane, odd level counts and stretched levels: the solve converges to ptol in a
+handful of corrections, and the fields agree with the FP64 path's within the
+mixed form's bars (1e-6 for p, whose right-hand side FP32 sources perturb;
+1e-5 for the others).
+"""
+import numpy as np
+import pytest
+
+from helpers import cases, live_mask_p, relerr
+
+pytestmark = pytest.mark.gpu
+
+
+def _steps(dcm, c, precision, nsteps=2, graphs=1):
+    core = dcm.DynamicalCore(c.grid)
+    core.solver_graphs(graphs)
+    core.upload_state(c.state, c.dt, ptol=c.ptol, kord=c.kord, precision=precision)
+    core.driver_start()
+    st = [core.step(1) for _ in range(nsteps)]
+    f = core.download_state()
+    core.close()
+    return st, f
+
+
+def _agree(c, f32, f64):
+    m = live_mask_p(c.grid)
+    p32, p64 = f32["p"][m], f64["p"][m]
+    assert relerr(p32 - p32.mean(), p64 - p64.mean()) <= 1e-6
+    for n in ("u", "v", "w", "th"):
+        assert relerr(f32[n], f64[n]) <= 1e-5, n
+
+
+SHAPES = [(64, 64, 48), (96, 60, 33), (97, 37, 61), (22, 91, 70), (26, 45, 128), (34, 127, 129),
+          (320, 14, 40), (1, 640, 210), (800, 1, 257), (128, 9, 300)]
+
+
+@pytest.mark.parametrize("shape", SHAPES)
+def test_direct_corrections_match_the_fp64_path(dcm, shape):
+    ip, jp, kp = shape
+    c = cases.warm_bubble(ip=ip, jp=jp, kp=kp, dxyz=50.0, radius=400.0, zc=500.0, seed=61)
+    st, f32 = _steps(dcm, c, 1)
+    for s in st:
+        assert s.err_last < c.ptol and 1 <= s.iters_last <= 5 and s.updates_last == s.iters_last
+    _agree(c, f32, _steps(dcm, c, 0)[1])
+
+
+def test_graph_and_host_driven_corrections_agree(dcm):
+    c = cases.warm_bubble(ip=90, jp=50, kp=41, dxyz=50.0, radius=400.0, zc=500.0, seed=62)
+    (sa, a), (sb, b) = (_steps(dcm, c, 1, graphs=g) for g in (1, 0))
+    assert [s.iters_last for s in sa] == [s.iters_last for s in sb]
+    for n in ("u", "v", "w", "th", "p"):
+        assert np.array_equal(a[n], b[n]), n
+
+
+def _with_spacing(g, axis, f):
+    """The grid with its spacings along one axis (name "x" or "z") scaled by f."""
+    for n in ("d" + axis, "d" + axis + "n"):
+        setattr(g, n, getattr(g, n) * f)
+    return g
+
+
+@pytest.mark.parametrize("axis", ["z", "x"])
+def test_stretched_spacings(dcm, axis):
+    """Stretched levels keep the direct corrections (the tridiagonal systems
+    take any spacing); uneven horizontal spacings take the FP32 iterations."""
+    c = cases.warm_bubble(ip=72, jp=64, kp=40, dxyz=50.0, radius=400.0, zc=500.0, seed=63)
+    n = len(getattr(c.grid, "d" + axis))
+    q = np.arange(n) / (n - 1.0)
+    _with_spacing(c.grid, axis,
+                  1.0 + 0.5 * q if axis == "z" else 1.0 + 0.1 * np.sin(2 * np.pi * q))
+    st, f32 = _steps(dcm, c, 1)
+    assert all(s.err_last < c.ptol for s in st)
+    assert all(s.iters_last <= 5 for s in st) if axis == "z" else \
+        all(s.iters_last > 5 for s in st)
+    _agree(c, f32, _steps(dcm, c, 0)[1])
+
+
+def test_limits_of_the_direct_corrections(dcm):
+    """itmax and the round budget bound the corrections as they bound the
+    iterations, with the same statuses."""
+    c = cases.warm_bubble(ip=64, jp=64, kp=48, dxyz=50.0, radius=400.0, zc=500.0, seed=64)
+    core = dcm.DynamicalCore(c.grid)
+    try:
+        def fresh(itmax=9999):
+            core.upload_state(c.state, c.dt, ptol=c.ptol, kord=c.kord, precision=1, itmax=itmax)
+            core.driver_start()
+        for itmax, rounds, status in ((1, 0, dcm.DCM_E_NOCONV), (9999, 1, dcm.DCM_E_TIMEOUT)):
+            fresh(itmax)
+            core.solver_limits(max_rounds=rounds)
+            with pytest.raises(dcm.DCMError) as e:
+                core.step(1)
+            assert e.value.status == status
+        core.solver_limits()
+        fresh()
+        assert core.step(1).err_last < c.ptol
+    finally:
+        core.close()
