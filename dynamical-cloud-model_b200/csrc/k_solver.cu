@@ -1222,6 +1222,10 @@ static void precond3(const SolverArgs& a, const Coef<float>& c, const SolverBufs
 
 // programmatic edges inside the graph-driven iterations (probed once)
 static int g_pdl_graphs = 0;
+// clusters of 16 blocks for the small solve (asked once: they need an SM group
+// with 16 free SMs)
+static int g_cluster16 = 0;
+static bool probe_cluster16();
 static bool probe_pdl_graphs();
 
 void solver_init() {
@@ -1236,7 +1240,10 @@ void solver_init() {
     cudaFuncSetAttribute(k_precond3<1, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          sm1m);
     static std::once_flag probed;  // handles may be created from several threads
-    std::call_once(probed, [] { g_pdl_graphs = probe_pdl_graphs() ? 1 : 0; });
+    std::call_once(probed, [] {
+        g_pdl_graphs = probe_pdl_graphs() ? 1 : 0;
+        g_cluster16 = probe_cluster16() ? 1 : 0;
+    });
 }
 
 bool solver_pdl_available() { return g_pdl_graphs != 0; }
@@ -1760,6 +1767,276 @@ __global__ void __launch_bounds__(SMALL_THREADS, 1)
     cl.sync();  // no block leaves while another may still read its partials
 }
 
+// The same solve with one point per thread (n <= SMALL_CL * SMALL_THREADS, the
+// default bound): every vector of the recursion is a register of its point's
+// thread, and only the operand of an operator application is exchanged, through
+// distributed shared memory.  The passes are bound by latency, so what counts
+// is that a neighbour value costs a shared-memory read (within the block, or
+// the neighbour block's for the few at its edges) instead of an L2 read behind
+// a barrier that has to flush stores to global memory.  Two exchange buffers
+// make one cluster barrier per pass enough: 11 per iteration, as above.  The
+// arithmetic is k_bicgstab_small's, statement by statement.  128 x 1 x 64
+// (the shear layer, steps 2..30), per iteration: k_bicgstab_small 28.4 us;
+// this on 8 blocks of 1024 threads about 18 us (the vectors spill at 64
+// registers); on 16 blocks of 512 threads 10.9 us, taken wherever the device
+// can place such a cluster.
+__device__ __forceinline__ unsigned smem_addr(const void* p) {
+    return (unsigned)__cvta_generic_to_shared(p);
+}
+// the address of this block's shared `a` in block `rank` of the cluster
+__device__ __forceinline__ unsigned cluster_addr(unsigned a, int rank) {
+    unsigned r;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ double cluster_ld(unsigned a) {
+    double v;
+    asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(a) : "memory");
+    return v;
+}
+__device__ __forceinline__ double shared_ld(unsigned a) {
+    double v;
+    asm volatile("ld.shared.f64 %0, [%1];" : "=d"(v) : "r"(a) : "memory");
+    return v;
+}
+__device__ __forceinline__ void cluster_st(unsigned a, double v) {
+    asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(a), "d"(v) : "memory");
+}
+
+template <int NT, int CL>
+__global__ void __launch_bounds__(NT, 1)
+    k_bicgstab_point(SolverArgs a, SmallOp op, double* __restrict__ x,
+                     const double* __restrict__ b, SolverScalars* S, int max_rounds) {
+    __shared__ double ex[2][NT];      // the exchanged operand, two buffers
+    __shared__ double part[2][2][256];  // [buffer][sum][warp of the cluster]
+    __shared__ double tot[2];
+    namespace cg = cooperative_groups;
+    cg::cluster_group cl = cg::this_cluster();
+    const Dims& d = a.d;
+    const int n = d.ip * d.jp * d.kp;
+    const int rank = (int)cl.block_rank();
+    const int tid = threadIdx.x;
+    const int q = rank * NT + tid;
+    const bool live = q < n;
+    int k = 1, j = 1, i = 1;
+    if (live) op.at(q, k, j, i);
+    const int o = d.at(k, j, i);
+    const double ae = ld(op.c.ae + i), aw = ld(op.c.aw + i), an = ld(op.c.an + j),
+                 as = ld(op.c.as + j), au = ld(op.c.au + k), ad = ld(op.c.ad + k);
+    const double ap = op.ap(k, j, i);
+    // the shared addresses of the six neighbours' operands: in this block's own
+    // window where the bit of `own` is set, else in the owning block's; a
+    // mirrored k neighbour is the point itself
+    const unsigned ex0 = smem_addr(&ex[0][0]), exb = NT * sizeof(double);
+    unsigned own = 0;
+    auto where = [&](int bit, int kk, int jj, int ii) -> unsigned {
+        const int qq = live ? (kk - 1) + d.kp * ((jj - 1) + d.jp * (ii - 1)) : q;
+        const int r = qq / NT;
+        const unsigned at = ex0 + (qq % NT) * (unsigned)sizeof(double);
+        if (r == rank) {
+            own |= 1u << bit;
+            return at;
+        }
+        return cluster_addr(at, r);
+    };
+    const unsigned nw = where(0, k, j, i == 1 ? d.ip : i - 1),
+                   ne = where(1, k, j, i == d.ip ? 1 : i + 1),
+                   ns = where(2, k, j == 1 ? d.jp : j - 1, i),
+                   nn = where(3, k, j == d.jp ? 1 : j + 1, i),
+                   nd = where(4, k == 1 ? 1 : k - 1, j, i),
+                   nu = where(5, k == d.kp ? k : k + 1, j, i);
+    auto get = [&](int bit, unsigned at, int buf) -> double {
+        at += buf ? exb : 0u;
+        return (own >> bit) & 1u ? shared_ld(at) : cluster_ld(at);
+    };
+    int eb = 0;  // exchange buffer of the next operand
+    // publish v, and after the barrier A v at this point (mat_ax, :219-222)
+    auto publish = [&](double v) {
+        ex[eb][tid] = v;
+        cl.sync();
+        eb ^= 1;
+    };
+    auto ax = [&](double v) -> double {
+        const int u = eb ^ 1;
+        const double xw = get(0, nw, u), xe = get(1, ne, u), xs = get(2, ns, u),
+                     xn = get(3, nn, u), xd = get(4, nd, u), xu = get(5, nu, u);
+        return aw * xw + ae * xe + as * xs + an * xn + ad * xd + au * xu + ap * v + 0.0;
+    };
+    int pb = 0;
+    // sums over the cluster, bit for bit k_bicgstab_small's: every warp's sum
+    // goes to every block; then one warp adds the 32 sums of 1,024 points in
+    // that kernel's tree, for the eight such groups at once, and the groups in
+    // order.  The tree's first step adds lanes 16 apart and so on down; a lane
+    // keeps half of its groups at each of the first three steps.
+    auto total = [&](const double* __restrict__ q) -> double {
+        constexpr unsigned FULL = 0xffffffffu;
+        const int lane = tid & 31;
+        double g[8];
+#pragma unroll
+        for (int r = 0; r < 8; r++) g[r] = q[32 * r + lane];
+#pragma unroll
+        for (int h = 4; h >= 1; h >>= 1) {
+            const bool up = lane & (4 * h);
+#pragma unroll
+            for (int r = 0; r < h; r++) {
+                const double send = up ? g[r] : g[r + h], keep = up ? g[r + h] : g[r];
+                g[r] = keep + __shfl_xor_sync(FULL, send, 4 * h);
+            }
+        }
+        g[0] += __shfl_xor_sync(FULL, g[0], 2);
+        g[0] += __shfl_xor_sync(FULL, g[0], 1);
+        double t = 0.0;
+#pragma unroll
+        for (int r = 0; r < 8; r++) t += __shfl_sync(FULL, g[0], 4 * r);
+        return t;
+    };
+    auto send = [&](int s, double v) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+        if ((tid & 31) < CL)
+            cluster_st(cluster_addr(smem_addr(&part[pb][s][rank * (NT / 32) + (tid >> 5)]),
+                                    tid & 31), v);
+    };
+    auto csum2 = [&](double& u, double& v) {
+        send(0, u);
+        send(1, v);
+        cl.sync();
+        if (tid < 64) {  // a warp per sum
+            const double t = total(part[pb][tid >> 5]);
+            if ((tid & 31) == 0) tot[tid >> 5] = t;
+        }
+        __syncthreads();
+        u = tot[0];
+        v = tot[1];
+        pb ^= 1;
+    };
+    auto csum1 = [&](double v) -> double {
+        send(0, v);
+        cl.sync();
+        if (tid < 32) {
+            const double t = total(part[pb][0]);
+            if (tid == 0) tot[0] = t;
+        }
+        __syncthreads();
+        pb ^= 1;
+        return tot[0];
+    };
+    // precondition (:241-270): s = q/a_p, three Jacobi sweeps
+    auto precondition = [&](double qv) -> double {
+        double s = qv / ap;
+#pragma unroll 1
+        for (int sweep = 0; sweep < 3; sweep++) {
+            publish(s);
+            s = s + (qv - ax(s)) / ap;
+        }
+        return s;
+    };
+    // ---- set-up (:367-383)
+    double xv = live ? x[o] : 0.0;
+    const double bv = live ? b[o] : 0.0;
+    publish(xv);
+    double rv = live ? bv - ax(xv) : 0.0;
+    const double crv = rv;
+    double pv = 0.0, v1 = 0.0;
+    double bb = bv * bv, rr = rv * rv;
+    csum2(bb, rr);
+    double sc = sqrt(bb);
+    sc = sc > a.sc_floor ? sc : a.sc_floor;  // :370-371
+    double err = sc > 0.0 ? sqrt(rr) / sc : 0.0;
+    int status = 0, it = 0, early = 0;
+    double rho = 0.0, alf = 1.0, omg = 1.0, nrm = 1.0, bet = 0.0, tt = 0.0, ts = 0.0;
+    double rc = rr;
+    if (err < a.tol) {
+        early = 1;  // :382-383
+    } else if (!(err == err)) {
+        status = DCM_E_NONFINITE;
+    } else {
+        for (it = 1;; it++) {
+            if (it > max_rounds) {
+                status = DCM_E_TIMEOUT;
+                it = it - 1;
+                break;
+            }
+            rho = rc;                                // :391
+            bet = (rho / nrm) * (alf / omg);         // :392
+            pv = precondition(rv - bet * (omg * v1)) + bet * pv;  // :393-397
+            publish(pv);
+            v1 = ax(pv);                             // :399-400
+            nrm = csum1(live ? crv * v1 : 0.0);      // :401
+            alf = rho / nrm;                         // :403
+            const double sv = rv - alf * v1;         // :404
+            const double cs = precondition(sv);      // :405-407
+            publish(cs);
+            const double tv = ax(cs);                // :408-409
+            double t2 = live ? tv * tv : 0.0, t3 = live ? tv * sv : 0.0;
+            csum2(t2, t3);
+            tt = t2;                                 // :410
+            ts = t3;                                 // :411
+            omg = ts / tt;                           // :412
+            if (fabs(omg) < a.tiny) {                // :414-417
+                status = DCM_E_BREAKDOWN;
+                break;
+            }
+            xv = xv + alf * pv + omg * cs;           // :419
+            rv = sv - omg * tv;                      // :420
+            double r2s = live ? rv * rv : 0.0, rcs = live ? rv * crv : 0.0;
+            csum2(r2s, rcs);
+            rc = rcs;
+            err = sqrt(r2s) / sc;                    // :423
+            nrm = rho;                               // :425
+            if (err < a.tol) break;                  // :428
+            if (!(err == err)) {
+                status = DCM_E_NONFINITE;
+                break;
+            }
+            if (it >= a.itmax) {
+                status = DCM_E_NOCONV;               // :431-434
+                break;
+            }
+        }
+        if (live) x[o] = xv;
+    }
+    if (tid == 0 && rank == 0) {
+        S->sc_err = sc;
+        S->err = err;
+        S->rho = rho;
+        S->alf = alf;
+        S->omg = omg;
+        S->bet = bet;
+        S->nrm = nrm;
+        S->tt = tt;
+        S->ts = ts;
+        S->it = it;
+        S->rounds = it;
+        S->status = status;
+        S->early = early;
+        S->done = 1;
+        S->pause = 0;
+        S->ru = 0;
+    }
+    cl.sync();  // no block leaves while another may still read its operand
+}
+
+static bool probe_cluster16() {
+    auto kern = k_bicgstab_point<512, 16>;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = 16;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(16);
+    cfg.blockDim = dim3(512);
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    int clusters = 0;
+    const bool good =
+        ok(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1)) &&
+        ok(cudaOccupancyMaxActiveClusters(&clusters, kern, &cfg)) && clusters > 0;
+    cudaGetLastError();
+    return good;
+}
+
 // the one-cluster solve applies (FP64, interior points <= w.small_max)
 template <typename T>
 static bool small_ok(const SolverWork<T>& w, const Dims& d) {
@@ -1821,8 +2098,22 @@ int solver_run(SolverWork<T>& w, const Dims& d, T* x, const T* b, const T* sw, c
                 cfg.stream = st;
                 cfg.attrs = at;
                 cfg.numAttrs = 1;
-                cudaLaunchKernelEx(&cfg, k_bicgstab_small, a, op, x, b, w.r, w.cr, w.p, w.v1, w.t,
-                                   w.sA, w.sB, w.rh, w.S, max_rounds);
+                // one point per thread where the cluster has as many
+                if (d.ip * d.jp * d.kp <= SMALL_CL * SMALL_THREADS) {
+                    if (g_cluster16) {
+                        at[0].val.clusterDim.x = 16;
+                        cfg.gridDim = dim3(16);
+                        cfg.blockDim = dim3(512);
+                        cudaLaunchKernelEx(&cfg, k_bicgstab_point<512, 16>, a, op, x, b, w.S,
+                                           max_rounds);
+                    } else {
+                        cudaLaunchKernelEx(&cfg, k_bicgstab_point<SMALL_THREADS, SMALL_CL>, a, op,
+                                           x, b, w.S, max_rounds);
+                    }
+                }
+                else
+                    cudaLaunchKernelEx(&cfg, k_bicgstab_small, a, op, x, b, w.r, w.cr, w.p, w.v1,
+                                       w.t, w.sA, w.sB, w.rh, w.S, max_rounds);
             }
             post_launch(st);
             if (w.graph && w.emit) return cudaPeekAtLastError() == cudaSuccess ? DCM_OK : DCM_E_CUDA;
