@@ -251,7 +251,7 @@ class DynamicalCore:
         self.lib = library()
         self.grid = grid
         self.shape = (grid.kp + 2, grid.jp + 2, grid.ip + 2)
-        self._state_keep = None
+        self._q_stack = None
         self._owned = _handle is None
         if _handle is not None:  # a member handle owned by an Ensemble
             self.h = _handle
@@ -493,15 +493,26 @@ class DynamicalCore:
         # su, sv, sw, sth, psrc and div are recomputed by the first step
         # (sources, the Poisson rhs, the divergence); left NULL they start at
         # zero on the device and nothing crosses PCIe for them
-        keep = []
+        # (nor is sq uploaded: the driver zeroes it each step)
         if nq:
-            qs = fortran_stack(state.q)
-            sq = fortran_stack([np.zeros(sh, order="F") for _ in range(nq)])
-            f.q, f.sq = qs.ctypes.data_as(_dp), sq.ctypes.data_as(_dp)
-            keep += [qs, sq]
+            f.q = self._stack_q(state.q, sh).ctypes.data_as(_dp)
         self._check(self.lib.dcm_state_upload(self.h, C.byref(cfg), C.byref(f)))
-        self._state_keep = keep
         self._nq = nq
+
+    def _stack_q(self, fields, sh):
+        """The q fields as consecutive blocks: a view when they are already,
+        else a copy into a stack this object keeps (its pages cost more to
+        touch for the first time than to fill again)."""
+        if isinstance(fields, np.ndarray) and fields.dtype == np.float64 and \
+                fields.shape[1:] == sh and all(a.flags.f_contiguous for a in fields) and \
+                _stacked(fields):
+            return fields
+        shape = (len(fields),) + sh
+        if self._q_stack is None or self._q_stack.shape != shape:
+            self._q_stack = empty_stack(len(fields), sh)
+        for dst, a in zip(self._q_stack, fields):
+            dst[...] = a
+        return self._q_stack
 
     def driver_start(self):
         self._check(self.lib.dcm_driver_start(self.h))
@@ -577,7 +588,7 @@ class DynamicalCore:
         for n, a in bars.items():
             setattr(f, n, _ptr(a))
         if self._nq:
-            q = fortran_stack([np.zeros(sh, order="F") for _ in range(self._nq)])
+            q = empty_stack(self._nq, sh)  # every element is written
             f.q = q.ctypes.data_as(_dp)
             out["q"] = q
         self._check(self.lib.dcm_state_download(self.h, C.byref(f)))
@@ -590,13 +601,16 @@ def _stacked(psi):
     return all(psi[q].ctypes.data == psi.ctypes.data + q * n * 8 for q in range(psi.shape[0]))
 
 
-def fortran_stack(fields):
-    """Stack nq Fortran-ordered fields into consecutive blocks, the memory
-    layout of a Fortran psi(:,:,:,1:nq)."""
-    nq = len(fields)
-    sh = fields[0].shape
+def empty_stack(nq, sh):
+    """nq uninitialised Fortran-ordered fields of shape sh as consecutive
+    blocks, the memory layout of a Fortran psi(:,:,:,1:nq)."""
     buf = np.empty((nq,) + sh[::-1], dtype=np.float64)  # C order of the reversed shape
-    out = buf.transpose(0, 3, 2, 1)  # each [q] is Fortran ordered with shape sh
+    return buf.transpose(0, 3, 2, 1)  # each [q] is Fortran ordered with shape sh
+
+
+def fortran_stack(fields):
+    """Stack nq Fortran-ordered fields into consecutive blocks."""
+    out = empty_stack(len(fields), fields[0].shape)
     for q, a in enumerate(fields):
         out[q][...] = a
     return out

@@ -11,6 +11,7 @@
 #include <string>
 #include <vector>
 
+#include "dcm_hostcopy.h"
 #include "dcm_internal.h"
 #include "dcm_prof.h"
 
@@ -81,7 +82,7 @@ struct dcm_handle {
     // named full-size scratch buffers
     std::vector<double*> slots;
     double* sg_lamsq = nullptr;  // lamsq of dcm_calculate_subgrid_3d (kp+2)
-    double* dense_stage = nullptr;  // one field in the host layout (uploads)
+    double* dense_stage = nullptr;  // one field in the host layout (copies)
     int first_call = 1;  // bicgstab_first, dynamics.f90:17
 
     // FP32 copies for the mixed-precision form
@@ -206,13 +207,32 @@ enum {
 // re-pitched (and converted to TO) on the device: a pitched 2-D host-to-device
 // copy of 1 KB rows ran at a sixth of the rate of the contiguous one.  The
 // stream orders the next field's copy into the stage after this kernel.
+int dense_stage(dcm_handle* h) {
+    if (!h->dense_stage) CK(cudaMalloc(&h->dense_stage, h->nh * sizeof(double)));
+    return DCM_OK;
+}
+
 template <typename TO>
 int upload_field(dcm_handle* h, TO* dst, const double* src) {
     if (!src) return DCM_OK;
-    if (!h->dense_stage) CK(cudaMalloc(&h->dense_stage, h->nh * sizeof(double)));
-    CK(cudaMemcpyAsync(h->dense_stage, src, h->nh * sizeof(double), cudaMemcpyHostToDevice,
-                       h->st));
+    const int rc = dense_stage(h);
+    if (rc != DCM_OK) return rc;
+    CK(hostcopy_h2d(h->dense_stage, src, h->nh * sizeof(double), h->st));
     launch_repitch<TO>(h->hd, h->d, dst, h->dense_stage, h->st);
+    return DCM_OK;
+}
+
+// A whole field back: re-pitched into the dense stage (and converted to FP64)
+// on the device, then one contiguous copy.  The 2-D copy of pitched rows this
+// replaces ran at 52.6 GB/s against 56.9 into page-locked memory, and at 12.8
+// into pageable memory.
+template <typename FROM>
+int download_field(dcm_handle* h, double* dst, const FROM* src) {
+    if (!dst) return DCM_OK;
+    const int rc = dense_stage(h);
+    if (rc != DCM_OK) return rc;
+    launch_unpitch<FROM>(h->hd, h->d, h->dense_stage, src, h->st);
+    CK(hostcopy_d2h(dst, h->dense_stage, h->nh * sizeof(double), h->st));
     return DCM_OK;
 }
 
@@ -230,10 +250,7 @@ int download(dcm_handle* h, double* dst, const double* src, size_t n = 0) {
         CK(cudaMemcpyAsync(dst, src, n * sizeof(double), cudaMemcpyDeviceToHost, h->st));
         return DCM_OK;
     }
-    const size_t w = (size_t)h->hd.K * sizeof(double);
-    CK(cudaMemcpy2DAsync(dst, w, src, (size_t)h->d.K * sizeof(double), w,
-                         (size_t)h->d.J * h->d.I, cudaMemcpyDeviceToHost, h->st));
-    return DCM_OK;
+    return download_field<double>(h, dst, src);
 }
 int sync(dcm_handle* h) {
     CK(cudaStreamSynchronize(h->st));
@@ -482,6 +499,7 @@ extern "C" int dcm_create(const dcm_grid* g, int device, dcm_handle** out) {
     if (direct_plan_build(d, ae, aw, an, as, au, ad, &h->direct) != DCM_OK)
         return cuda_fail(h, cudaGetLastError(), "direct solver tables");
     CK(cudaStreamSynchronize(h->st));
+    hostcopy_retain();
     *out = h;
     return DCM_OK;
 }
@@ -525,6 +543,7 @@ extern "C" int dcm_destroy(dcm_handle* h) {
     if (h->ev0) cudaEventDestroy(h->ev0);
     if (h->ev1) cudaEventDestroy(h->ev1);
     if (h->st) cudaStreamDestroy(h->st);
+    hostcopy_release();
     delete h;
     return DCM_OK;
 }
@@ -1230,11 +1249,12 @@ template <typename T>
 int get_field(dcm_handle* h, double* dst, const T* src, size_t n = 0) {
     if (!dst) return DCM_OK;
     if constexpr (std::is_same<T, double>::value) return download(h, dst, src, n);
+    if (!n) return download_field<T>(h, dst, src);
     double* stage = slot(h, S_STAGE);
     NEED(stage);
-    // the staging slot is reused by the next field; the stream orders that
-    // field's conversion after this copy, so no host synchronisation here
-    launch_convert<double, T>(n ? n : h->n, stage, src, h->st);
+    // the staging slot is reused by the next profile; the stream orders that
+    // one's conversion after this copy, so no host synchronisation here
+    launch_convert<double, T>(n, stage, src, h->st);
     RC(download(h, dst, stage, n));
     return DCM_OK;
 }
@@ -1378,6 +1398,22 @@ extern "C" int dcm_state_upload(dcm_handle* h, const dcm_config* cfg, const dcm_
                              (h->cfg.moisture ? h->cfg.nq : 0) ==
                                  (cfg->moisture ? cfg->nq : 0) &&
                              (h->cfg.viscous != 0) == (cfg->viscous != 0);
+    // an ensemble recaptures its steps where anything they captured changes: a
+    // pointer, or a configuration value (the forcing profiles are read from
+    // device memory that stays)
+    const dcm_config& o = h->cfg;
+    const bool same_steps =
+        same_layout && o.dt == cfg->dt && o.ptol == cfg->ptol &&
+        o.advection_scheme == cfg->advection_scheme && o.kord == cfg->kord &&
+        o.monotone == cfg->monotone && o.limiter == cfg->limiter && o.itmax == cfg->itmax &&
+        o.moisture == cfg->moisture && !cfg->moisture && o.thbase == cfg->thbase &&
+        o.thtop == cfg->thtop && o.inner_tol == cfg->inner_tol && o.precond == cfg->precond &&
+        o.precond_lo == cfg->precond_lo && o.z0 == cfg->z0 && o.z0th == cfg->z0th &&
+        o.forcing.damping_layer == cfg->forcing.damping_layer &&
+        o.forcing.forcing == cfg->forcing.forcing &&
+        o.forcing.divergence == cfg->forcing.divergence &&
+        o.forcing.forcing_tau == cfg->forcing.forcing_tau;
+    if (!same_steps) h->generation += 1;
     if (!same_layout) free_state(h);
     h->cfg = *cfg;
     h->cfg.lamsq = nullptr;  // copied to the device below; no host pointer is kept
@@ -1408,7 +1444,6 @@ extern "C" int dcm_state_upload(dcm_handle* h, const dcm_config* cfg, const dcm_
     h->t1 = h->t2 = 0.0;  // saved locals, :260
     h->refine_outer_total = 0;
     h->resident = true;
-    h->generation += 1;
     return sync(h);
 }
 

@@ -374,6 +374,9 @@ void launch_convert(size_t n, TO* to, const FROM* from, cudaStream_t st);
 // dense host-layout field (hd) -> pitched device field (d), converted to TO
 template <typename TO>
 void launch_repitch(const Dims& hd, const Dims& d, TO* dst, const double* src, cudaStream_t st);
+// pitched device field (d) of FROM -> dense FP64 layout (hd)
+template <typename FROM>
+void launch_unpitch(const Dims& hd, const Dims& d, double* dst, const FROM* src, cudaStream_t st);
 
 // psi (+/-) psi_1d(k) over the whole array (mpdata_3d_add :175-188)
 template <typename T>

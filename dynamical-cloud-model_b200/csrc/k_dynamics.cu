@@ -551,6 +551,32 @@ void launch_repitch(const Dims& hd, const Dims& d, TO* dst, const double* src, c
     const unsigned nb = (unsigned)std::min<size_t>((ncol + 7) / 8, 148 * 32);
     k_repitch<TO><<<nb, 256, 0, st>>>(hd, d, dst, src);
 }
+// the way back: pitched device columns (d.K levels) of FROM -> dense columns in
+// FP64, which one contiguous copy takes to the host
+template <typename FROM>
+__global__ void __launch_bounds__(256) k_unpitch(Dims hd, Dims d, double* __restrict__ dst,
+                                                 const FROM* __restrict__ src) {
+    const int lane = threadIdx.x & 31;
+    const size_t ncol = (size_t)hd.J * hd.I;
+    const size_t w0 = (blockIdx.x * (size_t)blockDim.x + threadIdx.x) >> 5;
+    const size_t nw = (gridDim.x * (size_t)blockDim.x) >> 5;
+    for (size_t col = w0; col < ncol; col += nw) {
+        const FROM* __restrict__ s = src + col * d.K;
+        double* __restrict__ t = dst + col * hd.K;
+        for (int k = lane; k < hd.K; k += 32) t[k] = (double)s[k];
+    }
+}
+template <typename FROM>
+void launch_unpitch(const Dims& hd, const Dims& d, double* dst, const FROM* src,
+                    cudaStream_t st) {
+    const size_t ncol = (size_t)hd.J * hd.I;
+    const unsigned nb = (unsigned)std::min<size_t>((ncol + 7) / 8, 148 * 32);
+    k_unpitch<FROM><<<nb, 256, 0, st>>>(hd, d, dst, src);
+}
+template void launch_unpitch<double>(const Dims&, const Dims&, double*, const double*,
+                                     cudaStream_t);
+template void launch_unpitch<float>(const Dims&, const Dims&, double*, const float*,
+                                    cudaStream_t);
 template void launch_repitch<double>(const Dims&, const Dims&, double*, const double*,
                                      cudaStream_t);
 template void launch_repitch<float>(const Dims&, const Dims&, float*, const double*,
