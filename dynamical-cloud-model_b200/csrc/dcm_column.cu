@@ -11,6 +11,7 @@
 // __syncwarp.  Reductions over k (minval, the positivity test's sum) are warp
 // shuffles.  All arithmetic is FP64 in the reference's order of terms.
 #include <algorithm>
+#include <cstring>
 
 #include "dcm_internal.h"
 
@@ -236,6 +237,157 @@ __global__ void __launch_bounds__(32 * COL_WARPS, 8) k_column_mpdata(ColArgs a) 
     for (int i = lane; i < a.nq * a.npsi; i += 32) gpsi[i] = psi[i];
 }
 
+// The sedimentation calls (kord 1, one halo level in psi): the column in
+// registers, level 1 + lane + 32 m of every field, so that neither the fields
+// nor the flux buffer pass through shared memory and no index arithmetic
+// remains (k_column_mpdata spends 3,000 warp instructions per column on the
+// same work, 77 % issue-bound).  A face's numerator
+//     N(k) = ((w + |w|) rhoa p(k) + (w - |w|) rhoa p(k+1)) dt
+// serves both levels it separates, and 1 / (2 dzn rhoan) is formed once per
+// column instead of two divisions per level, field and pass.
+template <int M, int NQ>
+__global__ void __launch_bounds__(32 * COL_WARPS) k_column_donor(ColArgs a) {
+    constexpr unsigned FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    const int c = blockIdx.x * COL_WARPS + (threadIdx.x >> 5);
+    if (c >= a.ncol) return;
+    const int kp = a.kp;
+    // level-0 views
+    double* __restrict__ gp = a.psi + (size_t)c * NQ * a.npsi;
+    const double* __restrict__ w = a.w + (size_t)c * a.nw + (a.l_h - 1);
+    const size_t mo = (size_t)c * a.mstride + (a.l_h - 1);
+    const double *dzn = a.dzn + mo, *rhoa = a.rhoa + mo, *rhoan = a.rhoan + mo;
+    const int ns = a.nsub ? max(a.nsub[c], 1) : 1;
+    const double dt = a.dt[c] / (double)ns;
+    double p[NQ][M], A[M], B[M], rd[M], lo[NQ], hi[NQ];
+#pragma unroll
+    for (int n = 0; n < NQ; n++) {
+#pragma unroll
+        for (int m = 0; m < M; m++) {
+            const int k = 1 + lane + 32 * m;
+            p[n][m] = k <= kp ? gp[(size_t)n * a.npsi + k] : 0.0;
+        }
+        lo[n] = gp[(size_t)n * a.npsi];  // halo levels 0 and kp + 1
+        hi[n] = gp[(size_t)n * a.npsi + kp + 1];
+    }
+#pragma unroll
+    for (int m = 0; m < M; m++) {
+        const int k = min(1 + lane + 32 * m, kp);
+        const double wk = w[k], ra = rhoa[k] * dt;
+        A[m] = (wk + fabs(wk)) * ra;
+        B[m] = (wk - fabs(wk)) * ra;
+        rd[m] = 1.0 / (2.0 * dzn[k] * rhoan[k]);
+    }
+    const double w0 = w[0], ra0 = rhoa[0] * dt;
+    const double A0 = (w0 + fabs(w0)) * ra0, B0 = (w0 - fabs(w0)) * ra0;
+    for (int s = 0; s < ns; s++) {
+        // positive definite (:507-516)
+        double mn[NQ];
+#pragma unroll
+        for (int n = 0; n < NQ; n++) {
+            double v = INFINITY;
+#pragma unroll
+            for (int m = 0; m < M; m++)
+                if (1 + lane + 32 * m <= kp) v = fmin(v, p[n][m]);
+            mn[n] = wmin(v);
+#pragma unroll
+            for (int m = 0; m < M; m++) p[n][m] -= mn[n];
+            lo[n] -= mn[n];
+            hi[n] -= mn[n];
+        }
+        double sum = 0.0;  // :518-529
+#pragma unroll
+        for (int m = 0; m < M; m++)
+            if (1 + lane + 32 * m <= kp) sum += p[0][m];
+        if (!(wsum(sum) < COL_SMALL)) {
+#pragma unroll
+            for (int n = 0; n < NQ; n++) {
+                // p(k+1): the next lane's, for lane 31 lane 0's next
+                double up[M], N[M];
+#pragma unroll
+                for (int m = 0; m < M; m++) up[m] = __shfl_sync(FULL, p[n][m], lane + 1);
+#pragma unroll
+                for (int m = 0; m < M; m++) {
+                    const int k = 1 + lane + 32 * m;
+                    double x = up[m];
+                    if (lane == 31) x = m + 1 < M ? up[m + 1 < M ? m + 1 : m] : hi[n];
+                    if (k == kp) x = hi[n];
+                    N[m] = A[m] * p[n][m] + B[m] * x;
+                }
+                // N(k-1): the lane below's, for lane 0 lane 31's before
+                const double first = __shfl_sync(FULL, p[n][0], 0);
+                double dn[M];
+#pragma unroll
+                for (int m = 0; m < M; m++) dn[m] = __shfl_sync(FULL, N[m], lane + 31);
+                const double N0 = A0 * lo[n] + B0 * first;
+#pragma unroll
+                for (int m = M - 1; m >= 0; m--) {
+                    const int k = 1 + lane + 32 * m;
+                    double below = dn[m];
+                    if (lane == 0) below = m > 0 ? dn[m > 0 ? m - 1 : 0] : N0;
+                    double fr = N[m] * rd[m], fl = below * rd[m];
+                    if (a.neumann == 1) {  // :65-67, in the reference's order
+                        if (k == 1) fl = fr;
+                        if (k == kp) fr = fl;
+                    } else if (a.neumann == 2) {  // :68-70
+                        if (k == 1) fl = -fr;
+                        if (k == kp) fr = -fl;
+                    }
+                    p[n][m] -= fr - fl;  // :73
+                }
+                lo[n] = hi[n] = 0.0;  // :755-761
+            }
+        }
+#pragma unroll
+        for (int n = 0; n < NQ; n++) {  // :775-777
+#pragma unroll
+            for (int m = 0; m < M; m++) p[n][m] += mn[n];
+            lo[n] += mn[n];
+            hi[n] += mn[n];
+        }
+    }
+#pragma unroll
+    for (int n = 0; n < NQ; n++) {
+        double* __restrict__ g = gp + (size_t)n * a.npsi;
+#pragma unroll
+        for (int m = 0; m < M; m++) {
+            const int k = 1 + lane + 32 * m;
+            if (k <= kp) g[k] = p[n][m];
+        }
+        if (lane == 0) {
+            g[0] = lo[n];
+            g[kp + 1] = hi[n];
+        }
+    }
+}
+
+// launches k_column_donor where it applies: up to 256 levels and three fields
+// (its registers), else false
+template <int M>
+static bool donor_m(const ColArgs& a, cudaStream_t st) {
+    const int nb = (a.ncol + COL_WARPS - 1) / COL_WARPS;
+    switch (a.nq) {
+        case 1: k_column_donor<M, 1><<<nb, 32 * COL_WARPS, 0, st>>>(a); return true;
+        case 2: k_column_donor<M, 2><<<nb, 32 * COL_WARPS, 0, st>>>(a); return true;
+        case 3: k_column_donor<M, 3><<<nb, 32 * COL_WARPS, 0, st>>>(a); return true;
+        default: return false;
+    }
+}
+static bool donor_launch(const ColArgs& a, cudaStream_t st) {
+    if (a.kord != 1 || a.r_h != 1) return false;
+    switch ((a.kp + 31) / 32) {
+        case 1: return donor_m<1>(a, st);
+        case 2: return donor_m<2>(a, st);
+        case 3: return donor_m<3>(a, st);
+        case 4: return donor_m<4>(a, st);
+        case 5: return donor_m<5>(a, st);
+        case 6: return donor_m<6>(a, st);
+        case 7:
+        case 8: return donor_m<8>(a, st);
+        default: return false;
+    }
+}
+
 }  // namespace
 
 // shape checks shared by both entry points; fills the launch shape
@@ -268,6 +420,7 @@ static int column_shape(int ncol, int kp, int nq, int l_h, int r_h, int metric_s
 }
 
 static bool column_launch(const ColArgs& a, int warps, size_t smem, cudaStream_t st) {
+    if (donor_launch(a, st)) return cudaPeekAtLastError() == cudaSuccess;
     if (smem > 48 * 1024 &&
         cudaFuncSetAttribute(k_column_mpdata, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)smem) != cudaSuccess)
@@ -302,6 +455,49 @@ extern "C" int dcm_mpdata_vec_1d_device(int ncol, int kp, int nq, int l_h, int r
     return column_launch(a, warps, smem, (cudaStream_t)stream) ? DCM_OK : DCM_E_CUDA;
 }
 
+// Device memory of the host-array calls, kept by the thread that makes them
+// (at most 32 MB, on one device) and freed when it ends: a cudaMalloc and the
+// cudaFree, which waits for the device, took most of a call of a few hundred
+// columns.  A thread's calls return after their last copy, so its next call
+// finds the memory free.
+namespace {
+constexpr size_t COL_KEEP = 32u << 20;
+constexpr size_t COL_PACK = 16u << 10;  // small arrays that go in one copy
+struct ColSpace {
+    char* p = nullptr;
+    size_t n = 0;
+    int device = -1;
+    void drop() {
+        int now = 0;
+        if (p && cudaGetDevice(&now) == cudaSuccess && cudaSetDevice(device) == cudaSuccess) {
+            cudaFree(p);
+            cudaSetDevice(now);
+        }
+        p = nullptr;
+        n = 0;
+    }
+    bool take(size_t want, char** out) {
+        int now = 0;
+        if (want > COL_KEEP || cudaGetDevice(&now) != cudaSuccess) return false;
+        if (want > n || now != device) {
+            drop();
+            device = now;
+            const size_t size = std::min(COL_KEEP, want + want / 2);
+            if (cudaMalloc(&p, size) != cudaSuccess) {
+                cudaGetLastError();
+                p = nullptr;
+                return false;
+            }
+            n = size;
+        }
+        *out = p;
+        return true;
+    }
+    ~ColSpace() { drop(); }
+};
+thread_local ColSpace col_space;
+}  // namespace
+
 extern "C" int dcm_mpdata_vec_1d(int ncol, int kp, int nq, int l_h, int r_h, const double* dt,
                                  const int* nsub, const double* dz, const double* dzn,
                                  const double* rhoa, const double* rhoan, int metric_stride,
@@ -324,10 +520,13 @@ extern "C" int dcm_mpdata_vec_1d(int ncol, int kp, int nq, int l_h, int r_h, con
     const size_t bytes_psi = (size_t)ncol * nq * npsi * sizeof(double);
     const size_t al = 256;
     auto up = [&](size_t b) { return (b + al - 1) / al * al; };
-    const size_t total = up(bytes_dt) + up(bytes_ns) + 4 * up(bytes_met) + up(bytes_w) +
-                         up(bytes_psi);
+    // [dt | nsub | four metrics] in one copy, then w, then psi
+    const size_t head = up(bytes_dt) + up(bytes_ns) + 4 * up(bytes_met);
     char* buf = nullptr;
-    if (cudaMalloc(&buf, total) != cudaSuccess) return DCM_E_CUDA;
+    ColSpace& space = col_space;
+    const size_t total = head + up(bytes_w) + up(bytes_psi);
+    const bool kept = space.take(total, &buf);
+    if (!kept && cudaMalloc(&buf, total) != cudaSuccess) return DCM_E_CUDA;
     size_t off = 0;
     auto take = [&](size_t b) {
         char* p = buf + off;
@@ -341,12 +540,24 @@ extern "C" int dcm_mpdata_vec_1d(int ncol, int kp, int nq, int l_h, int r_h, con
     double* d_w = (double*)take(bytes_w);
     double* d_psi = (double*)take(bytes_psi);
     const double* h_met[4] = {dz, dzn, rhoa, rhoan};
-    bool good = cudaMemcpy(d_dt, dt, bytes_dt, cudaMemcpyHostToDevice) == cudaSuccess;
-    if (good && nsub) good = cudaMemcpy(d_ns, nsub, bytes_ns, cudaMemcpyHostToDevice) == cudaSuccess;
-    for (int q = 0; q < 4 && good; q++)
-        good = cudaMemcpy(d_met[q], h_met[q], bytes_met, cudaMemcpyHostToDevice) == cudaSuccess;
-    if (good) good = cudaMemcpy(d_w, w, bytes_w, cudaMemcpyHostToDevice) == cudaSuccess;
-    if (good) good = cudaMemcpy(d_psi, psi, bytes_psi, cudaMemcpyHostToDevice) == cudaSuccess;
+    bool good = true;
+    auto send = [&](void* d, const void* h, size_t n) {
+        good = good && cudaMemcpyAsync(d, h, n, cudaMemcpyHostToDevice, 0) == cudaSuccess;
+    };
+    char packed[COL_PACK];
+    if (head <= COL_PACK) {
+        auto at = [&](const void* d) { return packed + ((const char*)d - buf); };
+        std::memcpy(at(d_dt), dt, bytes_dt);
+        if (nsub) std::memcpy(at(d_ns), nsub, bytes_ns);
+        for (int q = 0; q < 4; q++) std::memcpy(at(d_met[q]), h_met[q], bytes_met);
+        send(buf, packed, head);
+    } else {
+        send(d_dt, dt, bytes_dt);
+        if (nsub) send(d_ns, nsub, bytes_ns);
+        for (int q = 0; q < 4; q++) send(d_met[q], h_met[q], bytes_met);
+    }
+    send(d_w, w, bytes_w);
+    send(d_psi, psi, bytes_psi);
     a.monotone = monotone ? 1 : 0;
     a.dt = d_dt;
     a.nsub = nsub ? d_ns : nullptr;
@@ -358,6 +569,11 @@ extern "C" int dcm_mpdata_vec_1d(int ncol, int kp, int nq, int l_h, int r_h, con
     a.psi = d_psi;
     if (good) good = column_launch(a, warps, smem, 0);
     if (good) good = cudaMemcpy(psi, d_psi, bytes_psi, cudaMemcpyDeviceToHost) == cudaSuccess;
+    if (kept) {
+        // nothing of a failed call may still be reading the packed arrays
+        if (!good) cudaStreamSynchronize(0);
+        return good ? DCM_OK : DCM_E_CUDA;
+    }
     const bool freed = cudaFree(buf) == cudaSuccess;
     return good && freed ? DCM_OK : DCM_E_CUDA;
 }
