@@ -410,13 +410,14 @@ extern "C" int dcm_create(const dcm_grid* g, int device, dcm_handle** out) {
     const size_t I2 = g->ip + 2, J2 = g->jp + 2, K2 = g->kp + 2;
     // metrics block: dx dxn (I2) dy dyn (J2) dz dzn rhoa rhoan theta thetan (K2)
     //                ae aw (I2) an as (J2) au ad (K2)
+    //                1/dx 1/dxn (I2) 1/dy 1/dyn (J2) 1/dz 1/dzn (K2)
     // Each table starts FIELD_SHIFT elements past a multiple of FIELD_ALIGN,
     // so its element 1 is aligned like the fields' k = 1 (16-byte vector
     // loads of per-level coefficients); FIELD_PAD spare elements follow each.
     auto slot_len = [](size_t len) {
         return (len + FIELD_PAD + FIELD_ALIGN - 1) / FIELD_ALIGN * FIELD_ALIGN;
     };
-    const size_t nm = 4 * slot_len(I2) + 4 * slot_len(J2) + 8 * slot_len(K2) + FIELD_ALIGN;
+    const size_t nm = 6 * slot_len(I2) + 6 * slot_len(J2) + 10 * slot_len(K2) + FIELD_ALIGN;
     std::vector<double> hm(nm, 0.0);
     size_t o = FIELD_SHIFT;
     auto put = [&](const double* src, size_t len) {
@@ -445,12 +446,21 @@ extern "C" int dcm_create(const dcm_grid* g, int device, dcm_handle** out) {
     }
     const size_t o_ae = put(ae.data(), I2), o_aw = put(aw.data(), I2), o_an = put(an.data(), J2),
                  o_as = put(as.data(), J2), o_au = put(au.data(), K2), o_ad = put(ad.data(), K2);
+    auto put_r = [&](const double* src, size_t len) {
+        std::vector<double> r(len);
+        for (size_t q = 0; q < len; q++) r[q] = 1.0 / src[q];
+        return put(r.data(), len);
+    };
+    const size_t o_rx = put_r(g->dx, I2), o_rxn = put_r(g->dxn, I2), o_ry = put_r(g->dy, J2),
+                 o_ryn = put_r(g->dyn, J2), o_rz = put_r(g->dz, K2), o_rzn = put_r(g->dzn, K2);
     CK(cudaMalloc(&h->metric_block, nm * sizeof(double)));
     CK(cudaMemcpy(h->metric_block, hm.data(), nm * sizeof(double), cudaMemcpyHostToDevice));
     double* mb = h->metric_block;
     h->mt.dx = mb + o_dx; h->mt.dxn = mb + o_dxn; h->mt.dy = mb + o_dy; h->mt.dyn = mb + o_dyn;
     h->mt.dz = mb + o_dz; h->mt.dzn = mb + o_dzn; h->mt.rhoa = mb + o_ra; h->mt.rhoan = mb + o_rn;
     h->mt.theta = mb + o_th; h->mt.thetan = mb + o_thn;
+    h->mt.rdx = mb + o_rx; h->mt.rdxn = mb + o_rxn; h->mt.rdy = mb + o_ry;
+    h->mt.rdyn = mb + o_ryn; h->mt.rdz = mb + o_rz; h->mt.rdzn = mb + o_rzn;
     h->ae = mb + o_ae; h->aw = mb + o_aw; h->an = mb + o_an; h->as = mb + o_as;
     h->au = mb + o_au; h->ad = mb + o_ad;
     if (g->xg) h->h_xg.assign(g->xg, g->xg + I2);

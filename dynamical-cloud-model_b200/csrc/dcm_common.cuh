@@ -67,7 +67,22 @@ inline Dims make_dims_pitched(int ip, int jp, int kp) {
 template <typename T>
 struct Metrics {
     const T *dx, *dxn, *dy, *dyn, *dz, *dzn, *rhoa, *rhoan, *theta, *thetan;
+    // correctly rounded reciprocals of the spacings (FP64 metrics of a handle)
+    const T *rdx = nullptr, *rdxn = nullptr, *rdy = nullptr, *rdyn = nullptr, *rdz = nullptr,
+            *rdzn = nullptr;
 };
+
+// a / b from r, the correctly rounded 1 / b: the quotient's residual corrects
+// the product a r, which gives the correctly rounded quotient (P. Markstein,
+// "Computation of elementary functions on the IBM RISC System/6000 processor",
+// IBM J. Res. Dev. 34, 1990) in three FP64 operations, where the division
+// itself takes about twenty and bounds the kernels that form FP64 differences
+// of FP32 fields.  (An infinite a gives NaN, and a quotient below the normal
+// range may differ in its last bit.)
+__device__ __forceinline__ double div_r(double a, double b, double r) {
+    const double q = a * r;
+    return __fma_rn(__fma_rn(-q, b, a), r, q);
+}
 
 template <typename T>
 __device__ __forceinline__ T ld(const T* p) { return __ldg(p); }

@@ -39,40 +39,61 @@ void launch_exchange(const Dims& d, T* a, int mode, T lbc, T ubc, cudaStream_t s
 }
 
 // ---- horizontal means (+ divergence) --------------------------------------
-// threadIdx.x -> k (0..kp+1), threadIdx.y + blockIdx.y -> a fixed strided
-// set of (j,i) columns; per-(field, k) partials reduced in a fixed order by
-// the last block.  means layout: [field][k], k = 0..kp+1.
+// threadIdx.x -> k, threadIdx.y + blockIdx.y -> a fixed strided set of (j,i)
+// columns.  Blocks of the last blockIdx.x take the rows k = 0 and kp+1, the
+// others 32 levels each from k = 1, so that their rows start on a 32-byte
+// boundary.  The per-(field, k) partials are summed in block order by the last
+// block: a thread per (field, k), whose loads of different blocks' partials
+// are independent and coalesced over the threads (with a thread's partials
+// side by side in memory and one load at a time, that tail took most of the
+// kernel).  means layout: [field][k], k = 0..kp+1.
 
+// (five blocks per SM: at four the 640 blocks of 128 levels are just more than
+// one wave)
 template <typename T, int NF, typename D>
-__global__ void __launch_bounds__(256) k_means(Dims d, Metrics<D> mt, const T* f0, const T* f1,
-                                               const T* f2, const T* f3, T* __restrict__ means,
+__global__ void __launch_bounds__(256, 5) k_means(Dims d, Metrics<D> mt, const T* __restrict__ f0,
+                                               const T* __restrict__ f1,
+                                               const T* __restrict__ f2,
+                                               const T* __restrict__ f3, T* __restrict__ means,
                                                D* __restrict__ div, double* partials,
                                                unsigned int* ticket) {
     __shared__ double red[NF][BY][BX];
-    const int k = blockIdx.x * BX + threadIdx.x;
+    const bool ends = blockIdx.x == gridDim.x - 1;
+    const int k = ends ? (threadIdx.x == 0 ? 0 : threadIdx.x == 1 ? d.kp + 1 : d.kp + 2)
+                       : 1 + (int)(blockIdx.x * BX + threadIdx.x);
+    const bool in = ends ? k <= d.kp + 1 : k <= d.kp;
     const int ncol = d.ip * d.jp;
     const T* f[4] = {f0, f1, f2, f3};
     double acc[NF];
 #pragma unroll
     for (int q = 0; q < NF; q++) acc[q] = 0.0;
-    if (k <= d.kp + 1) {
-        for (int c = blockIdx.y * BY + threadIdx.y; c < ncol; c += gridDim.y * BY) {
-            const int j = 1 + c % d.jp, i = 1 + c / d.jp;
+    if (in) {
+        const int step = gridDim.y * BY, dj = step % d.jp, di = step / d.jp;
+        int c = blockIdx.y * BY + threadIdx.y, j = 1 + c % d.jp, i = 1 + c / d.jp;
+#pragma unroll 4
+        for (; c < ncol; c += step) {
             const int o = d.at(k, j, i);
 #pragma unroll
             for (int q = 0; q < NF; q++) acc[q] += (double)f[q][o];
-            if (div && k >= 1 && k <= d.kp) {
+            if (div && !ends) {
                 // divergence_calc, diagnostics.f90:144-146
                 // in D (FP64 for the mixed-precision form: the divergence check)
                 const T* u = f0;
                 const T* v = f1;
                 const T* w = f2;
                 const D rn = ld(mt.rhoan + k);
-                div[o] = rn * ((D)u[o] - (D)u[d.at(k, j, i - 1)]) / ld(mt.dx + i - 1) +
-                         rn * ((D)v[o] - (D)v[d.at(k, j - 1, i)]) / ld(mt.dy + j - 1) +
-                         (ld(mt.rhoa + k) * (D)w[o] - ld(mt.rhoa + k - 1) * (D)w[d.at(k - 1, j, i)]) /
-                             ld(mt.dz + k - 1);
+                div[o] = div_r(rn * ((D)u[o] - (D)u[d.at(k, j, i - 1)]), ld(mt.dx + i - 1),
+                               ld(mt.rdx + i - 1)) +
+                         div_r(rn * ((D)v[o] - (D)v[d.at(k, j - 1, i)]), ld(mt.dy + j - 1),
+                               ld(mt.rdy + j - 1)) +
+                         div_r(ld(mt.rhoa + k) * (D)w[o] -
+                                   ld(mt.rhoa + k - 1) * (D)w[d.at(k - 1, j, i)],
+                               ld(mt.dz + k - 1), ld(mt.rdz + k - 1));
             }
+            j += dj;
+            const int carry = j > d.jp;
+            j -= carry ? d.jp : 0;
+            i += di + carry;
         }
     }
 #pragma unroll
@@ -80,12 +101,12 @@ __global__ void __launch_bounds__(256) k_means(Dims d, Metrics<D> mt, const T* f
     __syncthreads();
     const unsigned int nbk = gridDim.x, nby = gridDim.y;
     const int K2 = d.kp + 2;
-    if (threadIdx.y == 0 && k <= d.kp + 1) {
+    if (threadIdx.y == 0 && in) {
 #pragma unroll
         for (int q = 0; q < NF; q++) {
             double s = 0.0;
             for (int y = 0; y < BY; y++) s += red[q][y][threadIdx.x];
-            partials[((size_t)q * K2 + k) * nby + blockIdx.y] = s;
+            partials[(size_t)blockIdx.y * (NF * K2) + q * K2 + k] = s;
         }
     }
     __shared__ bool s_last;
@@ -101,9 +122,10 @@ __global__ void __launch_bounds__(256) k_means(Dims d, Metrics<D> mt, const T* f
     const double area = (double)(d.ip * d.jp);
     const int tid = threadIdx.x + BX * threadIdx.y;
     for (int e = tid; e < NF * K2; e += BX * BY) {
-        const volatile double* p = partials + (size_t)e * nby;
+        const double* p = partials + e;
         double s = 0.0;
-        for (unsigned int b = 0; b < nby; b++) s += p[b];
+#pragma unroll 16
+        for (unsigned int b = 0; b < nby; b++) s += __ldcg(p + (size_t)b * (NF * K2));
         means[e] = (T)(s / area);  // diagnostics.f90:90-95
     }
     if (tid == 0) *ticket = 0u;
@@ -114,7 +136,7 @@ void launch_means_div(const Dims& d, const Metrics<D>& mt, const T* u, const T* 
                       const T* th, T* const* q, int nq, T* means, D* div, double* partials,
                       unsigned int* ticket, cudaStream_t st) {
     const int K2 = d.kp + 2;
-    const dim3 g((K2 + BX - 1) / BX, MEAN_GY), b(BX, BY);
+    const dim3 g((d.kp + BX - 1) / BX + 1, MEAN_GY), b(BX, BY);
     { ProfScope ps_(P_MEANS, st);
     k_means<T, 4, D><<<g, b, 0, st>>>(d, mt, u, v, w, th, means, div, partials, ticket);
     }
@@ -274,15 +296,11 @@ __global__ void __launch_bounds__(256) k_rhs(Dims d, Metrics<R> mt, const T* __r
     // the singular (periodic / Neumann) Poisson problem sums to zero to FP64
     // round-off and the FP64-refined solve stays consistent
     R r;
-    if (k >= 1) {
-        r = (((R)su[o] - (R)su[d.at(k, j, i - 1)]) / ld(mt.dx + i - 1) +
-             ((R)sv[o] - (R)sv[d.at(k, j - 1, i)]) / ld(mt.dy + j - 1) +
-             ((R)sw[o] - (R)sw[d.at(k - 1, j, i)]) / ld(mt.dz + k - 1));
-    } else {
-        r = (((R)su[o] - (R)su[d.at(0, j, i - 1)]) / ld(mt.dx + i - 1) +
-             ((R)sv[o] - (R)sv[d.at(0, j - 1, i)]) / ld(mt.dy + j - 1) +
-             ((R)sw[o] + (R)sw[d.at(1, j, i)]) / ld(mt.dz + 1));
-    }
+    const int kz = k >= 1 ? k - 1 : 1;
+    const R up = k >= 1 ? (R)sw[o] - (R)sw[d.at(k - 1, j, i)] : (R)sw[o] + (R)sw[d.at(1, j, i)];
+    r = (div_r((R)su[o] - (R)su[d.at(k, j, i - 1)], ld(mt.dx + i - 1), ld(mt.rdx + i - 1)) +
+         div_r((R)sv[o] - (R)sv[d.at(k, j - 1, i)], ld(mt.dy + j - 1), ld(mt.rdy + j - 1)) +
+         div_r(up, ld(mt.dz + kz), ld(mt.rdz + kz)));
     if (wo && k >= 1 && k <= d.kp)
         put_wo(rhs, d, k, j, i, r);
     else
@@ -387,9 +405,9 @@ __global__ void __launch_bounds__(256) k_momentum_step(Dims d, Metrics<T> mt, Me
     // pressure gradient in P (FP64 in the mixed-precision form, where p is
     // the refined FP64 solution), the rest in T
     const P pc = p[o];
-    const T gx = (T)((p[d.at(k, j, i + 1)] - pc) / (ld(mtp.dxn + i)));
-    const T gy = (T)((p[d.at(k, j + 1, i)] - pc) / (ld(mtp.dyn + j)));
-    const T gz = (T)((p[d.at(k + 1, j, i)] - pc) / (ld(mtp.dzn + k)));
+    const T gx = (T)div_r(p[d.at(k, j, i + 1)] - pc, ld(mtp.dxn + i), ld(mtp.rdxn + i));
+    const T gy = (T)div_r(p[d.at(k, j + 1, i)] - pc, ld(mtp.dyn + j), ld(mtp.rdyn + j));
+    const T gz = (T)div_r(p[d.at(k + 1, j, i)] - pc, ld(mtp.dzn + k), ld(mtp.rdzn + k));
     const T nu = zuo + ((su[o] - gx) * dt2) / ld(mt.rhoan + k);
     const T nv = zvo + ((sv[o] - gy) * dt2) / ld(mt.rhoan + k);
     const T nw = zwo + ((sw[o] - gz) * dt2) / ld(mt.rhoa + k);

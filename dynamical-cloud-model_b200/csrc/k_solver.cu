@@ -1048,17 +1048,24 @@ __global__ void __launch_bounds__(256) k_bicg_update(SolverArgs a, Coef<T> c,
 // --- after the solve: halo rows of x (dynamics.f90:437-442 or, after the
 //     early return, mat_ax's rows :203-211) and the driver's
 //     exchange_along_dim_wo(p) (driver_code.f90:506)
+// One thread per cell of the six faces of the interior (blockIdx.y: i, j, k
+// pair), which are all that have images; a cell on two faces is written twice
+// with the same values.
 template <typename T, typename TS>
 __global__ void __launch_bounds__(256) k_bicg_post(Dims d, T* __restrict__ x,
                                                    const TS* __restrict__ sw,
                                                    const T* __restrict__ dzn,
                                                    const SolverScalars* S, int wo) {
-    const int k = 1 + blockIdx.x * BX + threadIdx.x;
-    const int j = 1 + blockIdx.y * BY + threadIdx.y;
-    const int i = 1 + blockIdx.z;
-    if (k > d.kp || j > d.jp) return;
-    const int o = d.at(k, j, i);
-    const T v = x[o];
+    const int e = blockIdx.x * 256 + threadIdx.x;
+    const int pair = blockIdx.y;
+    const int n0 = pair == 2 ? d.jp : d.kp, n1 = pair == 0 ? d.jp : d.ip;
+    if (e >= 2 * n0 * n1) return;
+    const int side = e >= n0 * n1, f = e - side * n0 * n1;
+    const int c0 = 1 + f % n0, c1 = 1 + f / n0;
+    const int k = pair == 2 ? (side ? d.kp : 1) : c0;
+    const int j = pair == 0 ? c1 : pair == 1 ? (side ? d.jp : 1) : c0;
+    const int i = pair == 0 ? (side ? d.ip : 1) : c1;
+    const T v = x[d.at(k, j, i)];
     if (wo) put_wo(x, d, k, j, i, v);
     if (S->status != 0) return;
     if (S->early) {
@@ -1077,6 +1084,11 @@ __global__ void __launch_bounds__(256) k_bicg_post(Dims d, T* __restrict__ x,
                 x[d.at(0, jj, ii)] = v - (T)sw[d.at(0, jj, ii)] * dz0;
             }
     }
+}
+static dim3 post_grid(const Dims& d) {
+    const long long n = 2LL * std::max(std::max((long long)d.kp * d.jp, (long long)d.kp * d.ip),
+                                       (long long)d.ip * d.jp);
+    return dim3((unsigned)((n + 255) / 256), 3);
 }
 
 // --- host orchestration --------------------------------------------------------
@@ -2076,8 +2088,7 @@ int solver_run(SolverWork<T>& w, const Dims& d, T* x, const T* b, const T* sw, c
     auto post_launch = [&](cudaStream_t s) {
         if (post) {
             ProfScope ps(P_POST, s);
-            k_bicg_post<T, T><<<interior_grid(d, d.kp), dim3(BX, BY), 0, s>>>(d, x, sw, dzn, w.S,
-                                                                              wo);
+            k_bicg_post<T, T><<<post_grid(d), 256, 0, s>>>(d, x, sw, dzn, w.S, wo);
         }
     };
     if constexpr (std::is_same<T, double>::value) {
@@ -2501,7 +2512,7 @@ int refine_run(SolverWork<float>& wf, SolverWork<double>& wd, const Dims& d, dou
     auto finish = [&](cudaStream_t s) {
         k_ru_end<<<1, 1, 0, s>>>(wf.S, wd.S);
         ProfScope ps(P_POST, s);
-        k_bicg_post<double, float><<<gi, bl, 0, s>>>(d, x, sw, dzn, wd.S, 1);
+        k_bicg_post<double, float><<<post_grid(d), 256, 0, s>>>(d, x, sw, dzn, wd.S, 1);
     };
     // the iterations into the graph being captured on `s0`, their loop bodies
     // on the side streams lvl and lvl + 1:
