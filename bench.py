@@ -146,6 +146,13 @@ REF_ITER_PASSES = 39.0
 FUSED_JACOBI_PASSES = 3.5
 FUSED_REPLACED_PASSES = 11.5
 FUSED_ITER_PASSES = 25.0
+# A direct correction of the mixed form (in FP32 passes; FP64 fields count two):
+# four transforms and the tridiagonal systems, one field in and one out each,
+# the last transform into the FP64 pressure (1 + 4), and the FP64 residual
+# (p 2, b 2, r 1) that every correction and the start of a solve take.
+DIRECT_JACOBI_PASSES = 13.0 / 5.0
+DIRECT_SETUP_PASSES = 5.0
+DIRECT_ITER_PASSES = 18.0
 # With phase C's matvec as the fused kernel's fourth stage (launch shape
 # fuse = 2) phase C's launch also reads r, v1 and writes t (6 passes moved;
 # it replaces 11 + 4 = 15 algorithmic passes): per launch 5 moved and 13.5
@@ -368,7 +375,13 @@ def run_b200(args, rank, world, local_rank, dist):
     f_jac, f_rep, f_iter = ((FUSED_MV["jacobi"], FUSED_MV["replaced"], FUSED_MV["iter"])
                             if fuse_level == 2 else
                             (FUSED_JACOBI_PASSES, FUSED_REPLACED_PASSES, FUSED_ITER_PASSES))
+    # no matvec ran: every solve converged by direct corrections
+    direct = "matvec" not in classes
+    if direct:
+        fused, f_iter = False, DIRECT_ITER_PASSES
     dom_passes = f_jac if (fused and dom == "jacobi") else PASSES.get(dom, 0.0)
+    if direct and dom in ("jacobi", "setup"):
+        dom_passes = DIRECT_JACOBI_PASSES if dom == "jacobi" else DIRECT_SETUP_PASSES
     dom_bytes = dom_passes * N * w32
     dom_s = dom_ms / dom_n / 1e3 if dom_n else None
     # algorithmic bytes of one launch by the operator-fused model: a fused
@@ -451,7 +464,7 @@ def run_b200(args, rank, world, local_rank, dist):
     if rank != 0:
         return None
     extra = other_configs(args, local_rank) if (world == 1 and not args.no_extra) else None
-    sm32 = step_model(m32, w32, f_iter if fused else ITER_PASSES)
+    sm32 = step_model(m32, w32, f_iter if fused or direct else ITER_PASSES)
     sm64 = step_model(m64, 8.0, ITER_PASSES)
     acc_last = acc.get(str(args.accuracy_steps), {})
     details = {
@@ -459,23 +472,30 @@ def run_b200(args, rank, world, local_rank, dist):
                  "clocks": m64["clocks"], "step_model": sm64,
                  "kernel_ms": {k: round(v[0], 3) for k, v in m64["classes"].items()}},
         "mixed": {"tuned_launch_shape": m32["shape"], "step_model": sm32,
-                  "step_model_unfused_algorithm": step_model(m32, w32, ITER_PASSES),
+                  "step_model_unfused_algorithm":
+                      None if direct else step_model(m32, w32, ITER_PASSES),
                   "kernel_ms": {k: round(v[0], 3) for k, v in classes.items()},
                   "kernel_launches": {k: v[1] for k, v in classes.items()}},
         "mixed_reference_sweeps": {
             "value": m32ref["value"], "ms_per_step": m32ref["ms"] / args.steps,
             "bicgstab_iters_per_step": m32ref["iters"] / args.steps,
             "speedup_vs_fp64": m32ref["value"] / m64["value"],
-            "note": "the mixed form with the reference's unweighted Jacobi sweeps: the part "
-                    "of the speed-up that FP32 alone gives"},
+            "note": ("the mixed form with precond = 0; its solves take direct corrections, so "
+                     "neither run takes any sweeps" if direct else
+                     "the mixed form with the reference's unweighted Jacobi sweeps: the part "
+                     "of the speed-up that FP32 alone gives")},
         "accuracy_vs_fp64": acc,
-        "roofline_note": "achieved = the algorithmic bytes of the three Jacobi sweeps one fused "
+        "roofline_note": "achieved = the kernel class' field passes per launch time"
+                         if not (fused and dom == "jacobi") else
+                         "achieved = the algorithmic bytes of the three Jacobi sweeps one fused "
                          "launch applies (11.5 N-point FP32 passes, the operator-fused model) per "
                          "launch time; the fused kernel itself reads r/a_p, v1/a_p (and old p) "
                          "and writes p or cs, 3.5 passes, which min_bytes_frac counts",
         "e2e_host_ms": e2e.pop("host_ms"), "e2e_note": e2e.pop("note"),
-        "preconditioner": "FP32 iterations: Chebyshev-weighted Jacobi sweeps (3 sweeps, "
-                          "interval [0.05, 2]); FP64: the reference's 3 Jacobi sweeps",
+        "preconditioner": ("mixed form: direct corrections of the FP64 residual, counted as "
+                           "iterations; " if direct else
+                           "FP32 iterations: Chebyshev-weighted Jacobi sweeps (3 sweeps, "
+                           "interval [0.05, 2]); ") + "FP64: the reference's 3 Jacobi sweeps",
     }
     min_bytes = f_jac * N * w32 if (fused and dom == "jacobi") else dom_bytes
     return {
@@ -489,12 +509,15 @@ def run_b200(args, rank, world, local_rank, dist):
                  "step_frac_algorithm": step_model(m64, 8.0, REF_ITER_PASSES)["frac"]},
         "speedup_vs_fp64": m32["value"] / m64["value"],
         "iters_per_step": m32["iters"] / args.steps, "step_frac": sm32["frac"],
-        "step_frac_algorithm": step_model(m32, w32, REF_ITER_PASSES)["frac"],
+        "step_frac_algorithm":
+            None if direct else step_model(m32, w32, REF_ITER_PASSES)["frac"],
         "accuracy_vs_fp64_steps": args.accuracy_steps,
         "accuracy_vs_fp64": {n: float("%.3g" % v["max"]) for n, v in acc_last.items()},
         "config": bench_config(case, args),
         "parallelism": "replicas" if world > 1 else "single GPU",
-        "roofline": {"bound": "hbm", "kernel": dom + (" (fused preconditioner)" if fused else ""),
+        "roofline": {"bound": "hbm", "kernel": dom + (" (fused preconditioner)" if fused and dom == "jacobi" else
+                                      " (direct corrections)"
+                                      if direct and dom in ("jacobi", "setup") else ""),
                      "achieved": achieved_alg, "peak": peak, "unit": "GB/s",
                      "frac": (achieved_alg / peak) if achieved_alg else None,
                      "traffic": traffic, "peak_kind": peak_kind,

@@ -46,7 +46,7 @@ struct Coef {
 // ---- direct corrections of the mixed form's solve (k_direct.cu) -------------
 // The domains that take them, by interior points.  Measured per step (mixed
 // form, precond 1, iterations -> corrections): 97x75x61 7.4 -> 0.4 ms,
-// 256x256x128 34 -> 2.6 ms.  Smaller domains would gain too, but keep the
+// 256x256x128 34 -> 2.0 ms.  Smaller domains would gain too, but keep the
 // FP32 iterations: a step of 81x45x32 takes 4 ms, and the iteration counts
 // that dcm_step reports there are what the sweeps and launch shapes are
 // compared by.  Larger ones keep them because of p's additive constant, which

@@ -14,19 +14,19 @@
 // on with the BiCGSTAB iterations from there.
 //
 // Kernels per correction, each one pass in and one pass out of one FP32 field:
-//   k_fht      transform along y (r -> scratch)
-//   k_fht      transform along x (in place)
+//   k_fft      transform along y (r -> scratch)
+//   k_fft      transform along x (in place)
 //   k_zsolve   tridiagonal system of every mode's column (in place)
-//   k_fht      transform along x (in place)
-//   k_fht      transform along y, x += result (FP64)
+//   k_fft      inverse transform along x (in place)
+//   k_fft      inverse transform along y, x += result (FP64)
 //   k_dir_residual   r = b - A x, its norm, convergence and loop condition
 //
-// The transform is the discrete Hartley transform, sum a_j cas(2 pi m j / n):
-// real to real, its own inverse up to 1/n, and its basis vectors are
-// eigenvectors of a symmetric circulant, so a mode is one real number and a
-// field keeps its layout.  Two consecutive levels of a column make one
-// complex sequence, whose complex FFT Z gives both Hartley transforms
-// (Bracewell 1984):  H(m) = Re A - Im A with A = (Z(m) + conj Z(-m)) / 2.
+// Two consecutive levels of a column make one complex number, so a real field
+// transforms as complex sequences in its own layout and nothing is padded or
+// repacked: Z(m) = F1(m) + i F2(m) with the spectra F1, F2 of the two levels.
+// The operator's eigenvalues are even in m, and the pair Z(m), Z(-m) holds the
+// complex F1(m), F2(m), which k_zsolve forms in registers: their real and
+// imaginary parts are two real right-hand sides of the mode's one matrix.
 #include <algorithm>
 #include <cfloat>
 #include <cmath>
@@ -170,11 +170,11 @@ __device__ __forceinline__ void dft(float2 (&v)[R]) {
     }
 }
 
-// One Stockham pass of radix R over the C sequences of a tile (sequence c,
-// element m at [m C + c]): rows r0, r0 + rg, ... of butterflies per thread.
-template <int R, int C, bool FIRST, typename L>
+// One Stockham pass of radix R over the C sequences of a tile: rows r0, r0 +
+// rg, ... of butterflies per thread.  store(first element, stride, values).
+template <int R, bool FIRST, typename L, typename St>
 __device__ __forceinline__ void fft_pass(int n, int ns, const float2* __restrict__ tw, L load,
-                                         float2* __restrict__ dst, int c, int r0, int rg) {
+                                         St store, int r0, int rg) {
     const int nb = n / R;
     for (int b = r0; b < nb; b += rg) {
         float2 v[R];
@@ -187,19 +187,15 @@ __device__ __forceinline__ void fft_pass(int n, int ns, const float2* __restrict
             for (int t = 1; t < R; t++) v[t] = cmul_conj(v[t], __ldg(tw + t * step));
         }
         dft<R>(v);
-        const int o = (b - kk) * R + kk;
-#pragma unroll
-        for (int t = 0; t < R; t++) dst[(o + t * ns) * C + c] = v[t];
+        store((b - kk) * R + kk, ns, v);
     }
 }
 
 // a pass of any radix p (a prime factor above 13): each output is a sum of p
 // products
-template <int C>
-__device__ __forceinline__ void fft_pass_any(int p, int n, int ns,
-                                             const float2* __restrict__ tw,
-                                             const float2* __restrict__ src,
-                                             float2* __restrict__ dst, int c, int r0, int rg) {
+template <typename L, typename St>
+__device__ __forceinline__ void fft_pass_any(int p, int n, int ns, const float2* __restrict__ tw,
+                                             L load, St store, int r0, int rg) {
     const int nb = n / p;
     for (int o = r0; o < n; o += rg) {
         const int s = o / nb, b = o - s * nb, kk = b % ns;
@@ -207,24 +203,63 @@ __device__ __forceinline__ void fft_pass_any(int p, int n, int ns,
         float2 acc = make_float2(0.0f, 0.0f);
         int q = 0;
         for (int t = 0; t < p; t++) {
-            const float2 x = src[(b + t * nb) * C + c], w = __ldg(tw + q);
+            const float2 x = load(b + t * nb), w = __ldg(tw + q);
             acc.x += x.x * w.x + x.y * w.y;
             acc.y += x.y * w.x - x.x * w.y;
             q += q1;
             if (q >= n) q -= n;
         }
-        dst[((b - kk) * p + kk + s * ns) * C + c] = acc;
+        const float2 v[1] = {acc};
+        store((b - kk) * p + kk + s * ns, 0, v);
     }
 }
 
-template <int C, bool FIRST, typename L>
+// The first pass of such a radix, on the tile's elements in shared memory (x at
+// [m C]), where they are first replaced by the sums and differences of mirrored
+// pairs t, p - t: outputs s and p - s then share their products, a quarter of
+// them in all.  An item is a pair of outputs (s = 0: one).
+template <int C, typename St>
+__device__ __forceinline__ void fft_first_any(int p, int n, const float2* __restrict__ tw,
+                                              float2* x, St store, int r0, int rg) {
+    const int nb = n / p, h = (p - 1) / 2;
+    for (int e = r0; e < nb * h; e += rg) {
+        const int b = e % nb, t = 1 + e / nb;
+        const float2 u = x[(b + t * nb) * C], v = x[(b + (p - t) * nb) * C];
+        x[(b + t * nb) * C] = cadd(u, v);
+        x[(b + (p - t) * nb) * C] = csub(u, v);
+    }
+    __syncthreads();
+    for (int e = r0; e < nb * (h + 1); e += rg) {
+        const int b = e % nb, s = e / nb;
+        float2 a = x[b * C], d = make_float2(0.0f, 0.0f);
+        const int q1 = s * nb;  // < n
+        int q = 0;
+#pragma unroll 4
+        for (int t = 1; t <= h; t++) {
+            q += q1;
+            if (q >= n) q -= n;
+            const float2 u = x[(b + t * nb) * C], v = x[(b + (p - t) * nb) * C];
+            const float2 w = __ldg(tw + q);
+            a.x += w.x * u.x;
+            a.y += w.x * u.y;
+            d.x += w.y * v.x;
+            d.y += w.y * v.y;
+        }
+        const float2 lo[1] = {make_float2(a.x + d.y, a.y - d.x)};
+        const float2 hi[1] = {make_float2(a.x - d.y, a.y + d.x)};
+        store(b * p + s, 0, lo);
+        if (s) store(b * p + p - s, 0, hi);
+    }
+}
+
+template <bool FIRST, typename L, typename St>
 __device__ __forceinline__ void fft_pass_of(int radix, int n, int ns,
-                                            const float2* __restrict__ tw, L load,
-                                            float2* __restrict__ dst, int c, int r0, int rg) {
+                                            const float2* __restrict__ tw, L load, St store,
+                                            int r0, int rg) {
     switch (radix) {
-#define DCM_PASS(R)                                                   \
-    case R:                                                           \
-        fft_pass<R, C, FIRST>(n, ns, tw, load, dst, c, r0, rg);       \
+#define DCM_PASS(R)                                             \
+    case R:                                                     \
+        fft_pass<R, FIRST>(n, ns, tw, load, store, r0, rg);     \
         break;
         DCM_PASS(2) DCM_PASS(3) DCM_PASS(4) DCM_PASS(5) DCM_PASS(6) DCM_PASS(7) DCM_PASS(8)
         DCM_PASS(9) DCM_PASS(10) DCM_PASS(11) DCM_PASS(12) DCM_PASS(13) DCM_PASS(14)
@@ -234,15 +269,23 @@ __device__ __forceinline__ void fft_pass_of(int radix, int n, int ns,
     }
 }
 
-// ---- Hartley transform along one horizontal axis --------------------------------
+// ---- FFT along one horizontal axis -----------------------------------------------
 // A block transforms C pairs of levels (2 C consecutive levels) of one row or
 // column of the domain; every element of the tile is one C x 8 byte segment of
-// memory.  The first pass reads memory, the others go through two buffers in
-// shared memory.  OUT = 0: to dst; OUT = 1: x (FP64) += the transform (an
-// element that is not finite is left out, so that x stays usable).
-constexpr int FHT_THREADS = 256;
+// memory.  The first pass reads memory and the last writes it, so two radices
+// (n up to 256) meet in shared memory once; more take two buffers in turn.
+// The inverse is the forward transform with real and imaginary parts
+// exchanged.
+enum FftMode {
+    FFT_REAL = 0,  // forward, of a real field
+    FFT_FWD,       // forward, of complex pairs
+    FFT_INV,       // inverse, complex pairs
+    FFT_ADD        // inverse into a real field: x (FP64) += it; an element that
+                   // is not finite is left out, so that x stays usable
+};
+constexpr int FFT_THREADS = 256;
 
-struct FhtArgs {
+struct FftArgs {
     int n, nrad;
     int rad[DIRECT_MAX_RADICES];
     const float2* tw;  // n roots (cos, sin)(2 pi q / n)
@@ -250,85 +293,142 @@ struct FhtArgs {
     int kp, base;      // levels; index of (k, j, i) = (0, 1, 1)
 };
 
-template <int C, int OUT>
-__global__ void __launch_bounds__(FHT_THREADS) k_fht(FhtArgs a, const float* src, float* dst,
+template <int C, int MODE>
+__global__ void __launch_bounds__(FFT_THREADS, 3) k_fft(FftArgs a, const float* src, float* dst,
                                                      double* __restrict__ x) {
-    extern __shared__ float2 fht_buf[];
+    extern __shared__ float2 fft_buf[];
+    constexpr bool INV = MODE == FFT_INV || MODE == FFT_ADD;
     const int n = a.n, c = threadIdx.x % C, r0 = threadIdx.x / C;
-    constexpr int RG = FHT_THREADS / C;
-    float2* cur = fht_buf;
-    float2* nxt = fht_buf + n * C;
+    constexpr int RG = FFT_THREADS / C;
+    float2* cur = fft_buf + c;
+    float2* nxt = fft_buf + n * C + c;  // with three passes or more
     const int k0 = 1 + 2 * ((int)blockIdx.x * C + c);
     const bool one = k0 <= a.kp, both = k0 < a.kp;
     const int o0 = a.base + (int)blockIdx.y * a.batch + k0;
-    auto global = [&](int m) -> float2 {
+    auto swap = [](float2 v) { return INV ? make_float2(v.y, v.x) : v; };
+    // an odd last level is paired with a zero, in the scratch with the column's
+    // first padding element
+    auto get = [&](int m) -> float2 {
         const float* p = src + o0 + m * a.line;
-        if (both) return *reinterpret_cast<const float2*>(p);
-        return make_float2(one ? *p : 0.0f, 0.0f);
+        if (both || (MODE != FFT_REAL && one)) return swap(*reinterpret_cast<const float2*>(p));
+        return swap(make_float2(one ? *p : 0.0f, 0.0f));
     };
-    int ns = 1, q = 0;
-    if (a.nrad > 0 && a.rad[0] <= 16) {
-        fft_pass_of<C, true>(a.rad[0], n, 1, a.tw, global, cur, c, r0, RG);
-        ns = a.rad[0];
-        q = 1;
-    } else {
-        for (int m = r0; m < n; m += RG) cur[m * C + c] = global(m);
-    }
-    __syncthreads();
-    for (; q < a.nrad; q++) {
-        const int r = a.rad[q];
-        const float2* s = cur;
-        if (r <= 16)
-            fft_pass_of<C, false>(r, n, ns, a.tw, [&](int m) { return s[m * C + c]; }, nxt, c, r0,
-                                  RG);
-        else
-            fft_pass_any<C>(r, n, ns, a.tw, s, nxt, c, r0, RG);
-        ns *= r;
-        float2* t = cur;
-        cur = nxt;
-        nxt = t;
-        __syncthreads();
-    }
-    auto put = [&](int m, float h0, float h1) {
-        const int o = o0 + m * a.line;
-        if (OUT == 0) {
-            if (both)
-                *reinterpret_cast<float2*>(dst + o) = make_float2(h0, h1);
-            else if (one)
-                dst[o] = h0;
+    auto put = [&](int m, int stride, const auto& v) {
+        constexpr int R = sizeof(v) / sizeof(float2);
+        if constexpr (MODE != FFT_ADD) {
+#pragma unroll
+            for (int t = 0; t < R; t++)
+                if (one)
+                    *reinterpret_cast<float2*>(dst + o0 + (m + t * stride) * a.line) = swap(v[t]);
         } else {
-            if (!(fabsf(h0) <= FLT_MAX)) h0 = 0.0f;
-            if (!(fabsf(h1) <= FLT_MAX)) h1 = 0.0f;
-            if (both) {
-                double2 v = *reinterpret_cast<const double2*>(x + o);
-                v.x += (double)h0;
-                v.y += (double)h1;
-                *reinterpret_cast<double2*>(x + o) = v;
-            } else if (one) {
-                x[o] += (double)h0;
+            // x's values four at a time, so that their reads overlap
+            constexpr int G = R < 4 ? R : 4;
+#pragma unroll
+            for (int t = 0; t < R; t += G) {
+                double2 y[G];
+#pragma unroll
+                for (int g = 0; g < G; g++)
+                    if (t + g < R && one)
+                        y[g] = *reinterpret_cast<const double2*>(
+                            x + o0 + (m + (t + g) * stride) * a.line);
+#pragma unroll
+                for (int g = 0; g < G; g++) {
+                    if (t + g >= R || !one) continue;
+                    float2 h = swap(v[t + g < R ? t + g : 0]);
+                    if (!(fabsf(h.x) <= FLT_MAX)) h.x = 0.0f;
+                    if (!(fabsf(h.y) <= FLT_MAX)) h.y = 0.0f;
+                    double* w = x + o0 + (m + (t + g) * stride) * a.line;
+                    y[g].x += (double)h.x;
+                    y[g].y += (double)h.y;
+                    if (both)
+                        *reinterpret_cast<double2*>(w) = y[g];
+                    else
+                        *w = y[g].x;
+                }
             }
         }
     };
-    for (int m = r0; 2 * m <= n; m += RG) {
-        const int m2 = m ? n - m : 0;
-        const float2 z = cur[m * C + c], y = cur[m2 * C + c];
-        const float sx = 0.5f * (z.x + y.x), dx = 0.5f * (z.x - y.x);
-        const float sy = 0.5f * (z.y + y.y), dy = 0.5f * (z.y - y.y);
-        put(m, sx - dy, sy + dx);
-        if (m2 != m) put(m2, sx + dy, sy - dx);
+    int ns = 1, q = 0;
+    const bool small0 = a.nrad > 0 && a.rad[0] <= 16;
+    if (a.nrad == 1 && small0) {
+        fft_pass_of<true>(a.rad[0], n, 1, a.tw, get, put, r0, RG);
+        return;
+    }
+    if (small0) {
+        float2* d = cur;
+        fft_pass_of<true>(a.rad[0], n, 1, a.tw, get,
+                          [&](int m, int stride, const auto& v) {
+#pragma unroll
+                              for (int t = 0; t < (int)(sizeof(v) / sizeof(float2)); t++)
+                                  d[(m + t * stride) * C] = v[t];
+                          },
+                          r0, RG);
+        ns = a.rad[0];
+        q = 1;
+    } else {
+        for (int m = r0; m < n; m += RG) cur[m * C] = get(m);
+        if (a.nrad == 0) {  // n = 1
+            const float2 v[1] = {cur[0]};
+            if (r0 == 0) put(0, 0, v);
+            return;
+        }
+    }
+    __syncthreads();
+    if (q == 0) {
+        const int p = a.rad[0];
+        if (a.nrad == 1) {
+            fft_first_any<C>(p, n, a.tw, cur, put, r0, RG);
+            return;
+        }
+        float2* d = nxt;
+        fft_first_any<C>(p, n, a.tw, cur,
+                         [&](int m, int, const auto& v) { d[m * C] = v[0]; }, r0, RG);
+        ns = p;
+        q = 1;
+        nxt = cur;
+        cur = d;
+        __syncthreads();
+    }
+    for (; q < a.nrad; q++) {
+        const int r = a.rad[q];
+        const float2* s = cur;
+        auto load = [&](int m) { return s[m * C]; };
+        if (q + 1 == a.nrad) {
+            if (r <= 16)
+                fft_pass_of<false>(r, n, ns, a.tw, load, put, r0, RG);
+            else
+                fft_pass_any(r, n, ns, a.tw, load, put, r0, RG);
+            return;
+        }
+        float2* d = nxt;
+        auto store = [&](int m, int stride, const auto& v) {
+#pragma unroll
+            for (int t = 0; t < (int)(sizeof(v) / sizeof(float2)); t++)
+                d[(m + t * stride) * C] = v[t];
+        };
+        if (r <= 16)
+            fft_pass_of<false>(r, n, ns, a.tw, load, store, r0, RG);
+        else
+            fft_pass_any(r, n, ns, a.tw, load, store, r0, RG);
+        ns *= r;
+        nxt = cur;
+        cur = d;
+        __syncthreads();
     }
 }
 
 // ---- the tridiagonal systems along z ----------------------------------------------
-// One warp per column, V consecutive levels per lane.  Each lane eliminates
-// its inner levels (the partition method), the last level of every lane then
-// forms a 32-row tridiagonal system that cyclic reduction over the lanes
-// solves in five shuffle steps, and the inner levels follow by substitution.
-// A thread per column (the Thomas recurrence) would be a chain of 2 kp
-// dependent steps.  The horizontal mean mode is singular (Neumann at both
-// ends): it is integrated twice in FP64, with the additive constant that
-// leaves the sum of a_p dz-weighted values unchanged, which is the constant
-// Jacobi-preconditioned iterations leave unchanged too.
+// One warp per pair of modes m, -m, V consecutive levels per lane.  Their two
+// columns give the real and imaginary parts of the levels' spectra, two
+// right-hand sides of one matrix.  Each lane eliminates its inner levels (the
+// partition method), the last level of every lane then forms a 32-row
+// tridiagonal system that cyclic reduction over the lanes solves in five
+// shuffle steps, and the inner levels follow by substitution.  A thread per
+// column (the Thomas recurrence) would be a chain of 2 kp dependent steps.
+// The horizontal mean mode is singular (Neumann at both ends): it is
+// integrated twice in FP64, with the additive constant that leaves the sum of
+// a_p dz-weighted values unchanged, which is the constant Jacobi-preconditioned
+// iterations leave unchanged too.
 template <int V>
 __device__ __forceinline__ void zload(const float* __restrict__ p, int nvalid, float (&v)[V]) {
 #pragma unroll
@@ -386,71 +486,106 @@ __device__ __forceinline__ double warp_scan(double v) {  // inclusive
     return v;
 }
 
+// the mean mode's column D in place
+template <int V>
+__device__ __forceinline__ void mean_mode(const ZArgs& a, int k0, int nvalid, float (&D)[V]) {
+    double q[V], s = 0.0;
+#pragma unroll
+    for (int e = 0; e < V; e++) {
+        if (e < nvalid) s += a.w[k0 + e] * (double)D[e];
+        q[e] = s;
+    }
+    double before = warp_scan(s) - s, t = 0.0;
+#pragma unroll
+    for (int e = 0; e < V; e++) {
+        const double step = k0 + e < a.d.kp ? (q[e] + before) * a.g[k0 + e] : 0.0;
+        q[e] = t;
+        t += step;
+    }
+    before = warp_scan(t) - t;
+    double m = 0.0;
+#pragma unroll
+    for (int e = 0; e < V; e++) {
+        q[e] += before;
+        if (e < nvalid) m += a.l[k0 + e] * q[e];
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) m += __shfl_xor_sync(0xffffffffu, m, o);
+#pragma unroll
+    for (int e = 0; e < V; e++) D[e] = e < nvalid ? (float)(q[e] - m) : 0.0f;
+}
+
 template <int V>
 __global__ void __launch_bounds__(256) k_zsolve(ZArgs a, float* __restrict__ f) {
     constexpr unsigned FULL = 0xffffffffu;
     const Dims& d = a.d;
-    const int lane = threadIdx.x & 31, kp = d.kp;
+    const int lane = threadIdx.x & 31, kp = d.kp, ip = d.ip, jp = d.jp;
     const int k0 = 1 + V * lane;
     const int nvalid = max(0, min(V, kp - k0 + 1));
-    float au[V], ad[V], b0[V];
+    // levels of the columns in memory: an odd kp has one more (the imaginary
+    // part of its last pair)
+    const int nmem = max(0, min(V, kp + (kp & 1) - k0 + 1));
+    float au[V], ad[V];
 #pragma unroll
     for (int e = 0; e < V; e++) {
         const int k = k0 + e;
         au[e] = k < kp ? ld(a.au + k) : 0.0f;
         ad[e] = k > 1 && k <= kp ? ld(a.ad + k) : 0.0f;
-        b0[e] = -au[e] - ad[e];
     }
-    const int ncol = d.ip * d.jp, nw = gridDim.x * 8;
-    for (int col = blockIdx.x * 8 + (threadIdx.x >> 5); col < ncol; col += nw) {
-        const int i = col / d.jp, j = col - i * d.jp;
-        float* __restrict__ p = f + d.at(k0, 1 + j, 1 + i);
-        float D[V];
-        zload<V>(p, nvalid, D);
-#pragma unroll
-        for (int e = 0; e < V; e++) D[e] *= a.scale;
-        if (col == 0) {  // the whole warp
-            double q[V], s = 0.0;
-#pragma unroll
-            for (int e = 0; e < V; e++) {
-                if (e < nvalid) s += a.w[k0 + e] * (double)D[e];
-                q[e] = s;
-            }
-            double before = warp_scan(s) - s, t = 0.0;
+    // modes with 0 <= mx <= ip / 2; of the rows mx = 0 and mx = ip / 2, which
+    // hold their own partners, half
+    const int nmode = (ip / 2 + 1) * jp, nw = gridDim.x * 8;
+    for (int mode = blockIdx.x * 8 + (threadIdx.x >> 5); mode < nmode; mode += nw) {
+        const int mx = mode / jp, my = mode - mx * jp;
+        const int px = mx ? ip - mx : 0, py = my ? jp - my : 0;
+        if (px == mx && my > py) continue;
+        const bool self = px == mx && py == my;
+        float* __restrict__ p = f + d.at(k0, 1 + my, 1 + mx);
+        float* __restrict__ pp = f + d.at(k0, 1 + py, 1 + px);
+        float D[V], E[V];  // real and imaginary parts of the levels' spectra
+        zload<V>(p, nmem, D);
+        if (self) {
 #pragma unroll
             for (int e = 0; e < V; e++) {
-                const double step = k0 + e < kp ? (q[e] + before) * a.g[k0 + e] : 0.0;
-                q[e] = t;
-                t += step;
+                D[e] = e < nvalid ? D[e] * a.scale : 0.0f;
+                E[e] = 0.0f;
             }
-            before = warp_scan(t) - t;
-            double m = 0.0;
+        } else {
+            zload<V>(pp, nmem, E);
+            const float h = 0.5f * a.scale;
 #pragma unroll
-            for (int e = 0; e < V; e++) {
-                q[e] += before;
-                if (e < nvalid) m += a.l[k0 + e] * q[e];
+            for (int e = 0; e < V; e += 2) {  // (x, y) = Z(m), (z, w) = Z(-m)
+                const float x = D[e], y = D[e + 1], z = E[e], w = E[e + 1];
+                D[e] = h * (x + z);
+                D[e + 1] = h * (y + w);
+                E[e] = h * (y - w);
+                E[e + 1] = h * (z - x);
             }
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) m += __shfl_xor_sync(FULL, m, o);
-#pragma unroll
-            for (int e = 0; e < V; e++) D[e] = (float)(q[e] - m);
-            zstore<V>(p, nvalid, D);
+            for (int e = 0; e < V; e++)
+                if (e >= nvalid) D[e] = E[e] = 0.0f;
+        }
+        if (mode == 0) {
+            mean_mode<V>(a, k0, nvalid, D);
+            zstore<V>(p, nmem, D);
             continue;
         }
-        const float lam = ld(a.lx + i) + ld(a.ly + j);
+        const float lam = ld(a.lx + mx) + ld(a.ly + my);
         float A[V], C[V];
         // rows beyond kp: u = 0
 #pragma unroll
         for (int e = 0; e < V; e++) {
-            const float b = e < nvalid ? lam + b0[e] : 1.0f;
+            const float b = e < nvalid ? lam - ad[e] - au[e] : 1.0f;
             if (e < 2) {
                 const float r = __fdividef(1.0f, b);
                 D[e] *= r;
+                E[e] *= r;
                 A[e] = ad[e] * r;
                 C[e] = au[e] * r;
             } else {
                 const float r = __fdividef(1.0f, b - ad[e] * C[e - 1]);
                 D[e] = r * (D[e] - ad[e] * D[e - 1]);
+                E[e] = r * (E[e] - ad[e] * E[e - 1]);
                 A[e] = -r * ad[e] * A[e - 1];
                 C[e] = r * au[e];
             }
@@ -458,43 +593,62 @@ __global__ void __launch_bounds__(256) k_zsolve(ZArgs a, float* __restrict__ f) 
 #pragma unroll
         for (int e = V - 3; e >= 1; e--) {
             D[e] -= C[e] * D[e + 1];
+            E[e] -= C[e] * E[e + 1];
             A[e] -= C[e] * A[e + 1];
             C[e] = -C[e] * C[e + 1];
         }
         if (V > 2) {
             const float r = __fdividef(1.0f, 1.0f - C[0] * A[1]);
             D[0] = r * (D[0] - C[0] * D[1]);
+            E[0] = r * (E[0] - C[0] * E[1]);
             A[0] = r * A[0];
             C[0] = -r * C[0] * C[1];
         }
         // the last levels: first levels of this lane and the next eliminated
-        const float dn = __shfl_down_sync(FULL, D[0], 1), an = __shfl_down_sync(FULL, A[0], 1),
-                    cn = __shfl_down_sync(FULL, C[0], 1);
+        const float dn = __shfl_down_sync(FULL, D[0], 1), en = __shfl_down_sync(FULL, E[0], 1),
+                    an = __shfl_down_sync(FULL, A[0], 1), cn = __shfl_down_sync(FULL, C[0], 1);
         const float al = A[V - 1], cl = C[V - 1];
         float r = __fdividef(1.0f, 1.0f - al * C[0] - cl * an);
         float x = r * (D[V - 1] - al * D[0] - cl * dn);
+        float y = r * (E[V - 1] - al * E[0] - cl * en);
         float lo = -r * al * A[0], up = -r * cl * cn;
 #pragma unroll
         for (int s = 1; s < 32; s <<= 1) {
             // lo is 0 in the first s lanes and up in the last s, so what the
             // shuffles return there does not count
-            const float xm = __shfl_up_sync(FULL, x, s), lm = __shfl_up_sync(FULL, lo, s),
-                        um = __shfl_up_sync(FULL, up, s);
-            const float xp = __shfl_down_sync(FULL, x, s), lp = __shfl_down_sync(FULL, lo, s),
-                        upp = __shfl_down_sync(FULL, up, s);
+            const float xm = __shfl_up_sync(FULL, x, s), ym = __shfl_up_sync(FULL, y, s),
+                        lm = __shfl_up_sync(FULL, lo, s), um = __shfl_up_sync(FULL, up, s);
+            const float xp = __shfl_down_sync(FULL, x, s), yp = __shfl_down_sync(FULL, y, s),
+                        lp = __shfl_down_sync(FULL, lo, s), upp = __shfl_down_sync(FULL, up, s);
             r = __fdividef(1.0f, 1.0f - lo * um - up * lp);
             x = r * (x - lo * xm - up * xp);
+            y = r * (y - lo * ym - up * yp);
             lo = -r * lo * lm;
             up = -r * up * upp;
         }
-        float prev = __shfl_up_sync(FULL, x, 1);
-        if (lane == 0) prev = 0.0f;
-        const float u0 = D[0] - A[0] * prev - C[0] * x;
-        D[0] = u0;
+        float px1 = __shfl_up_sync(FULL, x, 1), py1 = __shfl_up_sync(FULL, y, 1);
+        if (lane == 0) px1 = py1 = 0.0f;
+        D[0] = D[0] - A[0] * px1 - C[0] * x;
+        E[0] = E[0] - A[0] * py1 - C[0] * y;
 #pragma unroll
-        for (int e = 1; e < V - 1; e++) D[e] = D[e] - A[e] * u0 - C[e] * x;
+        for (int e = 1; e < V - 1; e++) {
+            D[e] = D[e] - A[e] * D[0] - C[e] * x;
+            E[e] = E[e] - A[e] * E[0] - C[e] * y;
+        }
         D[V - 1] = x;
-        zstore<V>(p, nvalid, D);
+        E[V - 1] = y;
+        if (!self) {
+#pragma unroll
+            for (int e = 0; e < V; e += 2) {
+                const float re = D[e], rf = D[e + 1], im = E[e], in = E[e + 1];
+                D[e] = re - in;
+                D[e + 1] = im + rf;
+                E[e] = re + in;
+                E[e + 1] = rf - im;
+            }
+            zstore<V>(pp, nmem, E);
+        }
+        zstore<V>(p, nmem, D);
     }
 }
 
@@ -502,8 +656,9 @@ __global__ void __launch_bounds__(256) k_zsolve(ZArgs a, float* __restrict__ f) 
 // r = b - A x in FP64 (mat_ax, dynamics.f90:219-222), stored in FP32, with
 // ||r|| and, at the start of a solve, ||b||.  A warp holds 64 levels (one
 // 16-byte vector per lane) of one row and marches along i with the i - 1, i
-// and i + 1 columns in registers; the next plane's loads are issued before
-// this plane's arithmetic.
+// and i + 1 columns in registers.  (Loading the next plane ahead into
+// registers left two blocks per SM: 75 us against
+// 55 at 256 x 256 x 128; 235 MB, 36 us at the copy rate.)
 struct DirResidualArgs {
     Dims d;
     Coef<double> c;
@@ -517,7 +672,7 @@ struct DirResidualArgs {
 };
 
 template <bool FIRST>
-__global__ void __launch_bounds__(256) k_dir_residual(DirResidualArgs a, Red2 R,
+__global__ void __launch_bounds__(256, 4) k_dir_residual(DirResidualArgs a, Red2 R,
                                                       SolverScalars* S) {
     __shared__ double smem[64];
     const Dims& d = a.d;
@@ -538,22 +693,15 @@ __global__ void __launch_bounds__(256) k_dir_residual(DirResidualArgs a, Red2 R,
         const double au0 = ld(a.c.au + kl), au1 = ld(a.c.au + kl + 1), ad0 = ld(a.c.ad + kl),
                      ad1 = ld(a.c.ad + kl + 1);
         auto at = [](const double* p) { return *reinterpret_cast<const double2*>(p); };
-        double2 xw = at(x + KJ * (i0 == 1 ? ip : i0 - 1)), xc = at(x + KJ * i0),
-                xe = at(x + KJ * (i0 == ip ? 1 : i0 + 1)), xs = at(x + KJ * i0 + ds),
-                xn = at(x + KJ * i0 + dn), bv = at(bb + KJ * i0);
+        double2 xw = at(x + KJ * (i0 == 1 ? ip : i0 - 1)), xc = at(x + KJ * i0);
         for (int i = i0; i <= i1; i++) {
             const int o = KJ * i;
+            const double2 xe = at(x + KJ * (i == ip ? 1 : i + 1)), xs = at(x + o + ds),
+                          xn = at(x + o + dn), bv = at(bb + o);
             double prev = __shfl_up_sync(0xffffffffu, xc.y, 1);
             double next = __shfl_down_sync(0xffffffffu, xc.x, 1);
             if (lane == 0 && live && k0 > 1) prev = x[o - 1];
             if (lane == 31 && k0 + 2 <= kp) next = x[o + 2];
-            double2 xe2, xs2, xn2, b2;
-            if (i < i1) {
-                xe2 = at(x + KJ * (i + 1 == ip ? 1 : i + 2));
-                xs2 = at(x + o + KJ + ds);
-                xn2 = at(x + o + KJ + dn);
-                b2 = at(bb + o + KJ);
-            }
             const double ae = ld(a.c.ae + i), aw = ld(a.c.aw + i);
             const double sij = -ae - aw - an - as;
             if (k0 == 1) prev = xc.x;  // Neumann rows, :206-211
@@ -576,12 +724,6 @@ __global__ void __launch_bounds__(256) k_dir_residual(DirResidualArgs a, Red2 R,
             }
             xw = xc;
             xc = xe;
-            if (i < i1) {
-                xe = xe2;
-                xs = xs2;
-                xn = xn2;
-                bv = b2;
-            }
         }
     }
     block_reduce<R_SUM, 2>(acc, smem);
@@ -685,7 +827,12 @@ bool uniform(const std::vector<double>& a, const std::vector<double>& b, int n) 
 // sequences per tile: 16 (128-byte segments) while two buffers of a line
 // leave room for three blocks per SM, else 8
 int tile_pairs(int n) { return n <= 288 ? 16 : 8; }
-size_t fht_smem(int n) { return (size_t)2 * n * tile_pairs(n) * sizeof(float2); }
+// shared memory of a block: a buffer between two passes, two buffers for three
+// passes or more; a first pass of a large radix reads a buffer too
+size_t fft_smem(int n, int nrad, int first) {
+    const int meetings = nrad - 1 + (first > 16 ? 1 : 0);
+    return (size_t)(meetings > 1 ? 2 : 1) * n * tile_pairs(n) * sizeof(float2);
+}
 
 }  // namespace
 
@@ -702,8 +849,10 @@ int direct_plan_build(const Dims& d, const std::vector<double>& ae, const std::v
     if (points < DIRECT_MIN_POINTS || points > DIRECT_MAX_POINTS || d.kp > 32 * 16 ||
         !uniform(ae, aw, d.ip) || !uniform(an, as, d.jp))
         return DCM_OK;
-    for (int q = 0; q < 2; q++)
-        if (fht_smem(n[q]) > DIRECT_MAX_SMEM) return DCM_OK;
+    for (int q = 0; q < 2; q++) {
+        const std::vector<int> r = radices(n[q]);
+        if (fft_smem(n[q], (int)r.size(), r.empty() ? 0 : r[0]) > DIRECT_MAX_SMEM) return DCM_OK;
+    }
     for (int k = 1; k <= d.kp; k++)
         if (!(au[k] > 0.0 && ad[k] > 0.0)) return DCM_OK;
     // one block: per axis n roots (float2) and n eigenvalues, then the mean
@@ -762,17 +911,24 @@ int direct_plan_build(const Dims& d, const std::vector<double>& ae, const std::v
 
 void direct_init() {
     const int sm = (int)DIRECT_MAX_SMEM;
-    cudaFuncSetAttribute(k_fht<16, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
-    cudaFuncSetAttribute(k_fht<16, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
-    cudaFuncSetAttribute(k_fht<8, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
-    cudaFuncSetAttribute(k_fht<8, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
+    auto set = [&](auto kern) {
+        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
+    };
+    set(k_fft<16, FFT_REAL>);
+    set(k_fft<16, FFT_FWD>);
+    set(k_fft<16, FFT_INV>);
+    set(k_fft<16, FFT_ADD>);
+    set(k_fft<8, FFT_REAL>);
+    set(k_fft<8, FFT_FWD>);
+    set(k_fft<8, FFT_INV>);
+    set(k_fft<8, FFT_ADD>);
 }
 
-// the transform along axis 0 (x) or 1 (y); x non-null: added to it
-static void fht(const DirectPlan& P, const Dims& d, int axis, const float* src, float* dst,
-                double* x, cudaStream_t st) {
+// the transform along axis 0 (x) or 1 (y) (x: the field that FFT_ADD adds to)
+static void fft(const DirectPlan& P, const Dims& d, int axis, FftMode mode, const float* src,
+                float* dst, double* x, cudaStream_t st) {
     const AxisPlan& X = P.axis[axis];
-    FhtArgs a;
+    FftArgs a;
     a.n = X.n;
     a.nrad = X.nrad;
     std::copy(X.rad, X.rad + DIRECT_MAX_RADICES, a.rad);
@@ -783,20 +939,21 @@ static void fht(const DirectPlan& P, const Dims& d, int axis, const float* src, 
     a.base = d.at(0, 1, 1);
     const int C = tile_pairs(X.n);
     const dim3 g(((d.kp + 1) / 2 + C - 1) / C, axis == 0 ? d.jp : d.ip);
-    const size_t sm = fht_smem(X.n);
+    const size_t sm = fft_smem(X.n, X.nrad, X.rad[0]);
     ProfScope ps(P_JACOBI, st);
-    if (C == 16)
-        x ? k_fht<16, 1><<<g, FHT_THREADS, sm, st>>>(a, src, dst, x)
-          : k_fht<16, 0><<<g, FHT_THREADS, sm, st>>>(a, src, dst, x);
-    else
-        x ? k_fht<8, 1><<<g, FHT_THREADS, sm, st>>>(a, src, dst, x)
-          : k_fht<8, 0><<<g, FHT_THREADS, sm, st>>>(a, src, dst, x);
+    auto go = [&](auto kern) { kern<<<g, FFT_THREADS, sm, st>>>(a, src, dst, x); };
+    switch (mode) {
+        case FFT_REAL: C == 16 ? go(k_fft<16, FFT_REAL>) : go(k_fft<8, FFT_REAL>); break;
+        case FFT_FWD: C == 16 ? go(k_fft<16, FFT_FWD>) : go(k_fft<8, FFT_FWD>); break;
+        case FFT_INV: C == 16 ? go(k_fft<16, FFT_INV>) : go(k_fft<8, FFT_INV>); break;
+        case FFT_ADD: C == 16 ? go(k_fft<16, FFT_ADD>) : go(k_fft<8, FFT_ADD>); break;
+    }
 }
 
 void direct_correction(const DirectPlan& P, const Dims& d, const Coef<float>& c, const float* r,
                        float* work, double* x, cudaStream_t st) {
-    fht(P, d, 1, r, work, nullptr, st);
-    if (d.ip > 1) fht(P, d, 0, work, work, nullptr, st);
+    fft(P, d, 1, FFT_REAL, r, work, nullptr, st);
+    if (d.ip > 1) fft(P, d, 0, FFT_FWD, work, work, nullptr, st);
     {
         ZArgs z;
         z.d = d;
@@ -808,7 +965,7 @@ void direct_correction(const DirectPlan& P, const Dims& d, const Coef<float>& c,
         z.g = P.g;
         z.l = P.l;
         z.scale = (float)(1.0 / ((double)d.ip * d.jp));
-        const int nb = (d.ip * d.jp + 7) / 8;
+        const int nb = ((d.ip / 2 + 1) * d.jp + 7) / 8;
         const int g = std::min(nb, 148 * 16);
         ProfScope ps(P_JACOBI, st);
         if (d.kp <= 64)
@@ -820,8 +977,8 @@ void direct_correction(const DirectPlan& P, const Dims& d, const Coef<float>& c,
         else
             k_zsolve<16><<<g, 256, 0, st>>>(z, work);
     }
-    if (d.ip > 1) fht(P, d, 0, work, work, nullptr, st);
-    fht(P, d, 1, work, nullptr, x, st);
+    if (d.ip > 1) fft(P, d, 0, FFT_INV, work, work, nullptr, st);
+    fft(P, d, 1, FFT_ADD, work, nullptr, x, st);
 }
 
 void direct_residual(const Dims& d, const Coef<double>& c, const double* x, const double* b,
@@ -840,9 +997,10 @@ void direct_residual(const Dims& d, const Coef<double>& c, const double* x, cons
     a.cond = cond ? *cond : 0;
     a.use_cond = cond ? 1 : 0;
     dim3 g((d.kp + 63) / 64, (d.jp + BY - 1) / BY, 1);
-    // about four blocks per SM, each marching over at least 4 planes
+    // at most four blocks per SM (all resident), each marching over at least 4
+    // planes
     const int plane = g.x * g.y;
-    int want = std::max(1, std::min((d.ip + 3) / 4, (148 * 4 + plane - 1) / plane));
+    int want = std::max(1, std::min((d.ip + 3) / 4, 148 * 4 / plane));
     want = std::max(1, std::min(want, max_blocks / plane));
     a.ni = (d.ip + want - 1) / want;
     g.z = (d.ip + a.ni - 1) / a.ni;

@@ -1,9 +1,9 @@
-"""GPU checks of the mixed form's direct corrections (Hartley transforms along
-x and y, tridiagonal systems along z, in FP32, on the FP64 residual).
+"""GPU checks of the mixed form's direct corrections (transforms along x and y,
+tridiagonal systems along z, in FP32, on the FP64 residual).
 
 A step of domains above the size where they start, at transform lengths of
-every kind (powers of two, products of the other small radices, primes, a
-length whose tiles are narrower, 1), columns of one to sixteen levels per
+every kind (powers of two, products of the other small radices, primes alone
+and with other radices, a length whose tiles are narrower, 1), columns of one to sixteen levels per
 lane, odd level counts and stretched levels: the solve converges to ptol in a
 handful of corrections, and the fields agree with the FP64 path's within the
 mixed form's bars (1e-6 for p, whose right-hand side FP32 sources perturb;
