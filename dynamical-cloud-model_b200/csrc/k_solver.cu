@@ -117,6 +117,7 @@ struct SolverBufs {
     const void *x, *b, *r, *v1, *rh, *vh, *sin, *cr;
     void *out, *out2, *out3;
     int sweep;  // 1..3: which Jacobi sweep of the preconditioner a launch is
+    int back;   // a sweep that takes the i-planes from the last to the first
 };
 
 // q / a_p of the preconditioner input, formed from rh = r/a_p and vh = v1/a_p:
@@ -514,12 +515,14 @@ __device__ __forceinline__ void reduce_tail(const SolverArgs& a, double (&acc)[N
     }
 }
 
-// Sweeps (no reduction): one warp task per warp, grid (k-chunks, j/8, i).
-// Reducing kernels: persistent blocks, each warp strides over the warp tasks
-// and the block publishes one partial.
-template <typename T, int OP, int MODE, int V = KVec<T>::V, bool RM = false>
-__global__ void __launch_bounds__(256) k_sten(SolverArgs a, Coef<T> c, SolverBufs B, Red2 R,
-                                              SolverScalars* S) {
+// Sweeps (no reduction): one warp task per warp, grid (k-chunks, j/8, i), or
+// with PS persistent blocks.  Reducing kernels: persistent blocks, each warp
+// strides over the warp tasks and the block publishes one partial; their grid
+// is what is resident, so the order of their sums hangs on their register
+// count: only PS instances are given a least number of blocks.
+template <typename T, int OP, int MODE, int V = KVec<T>::V, bool RM = false, bool PS = false>
+__global__ void __launch_bounds__(256, PS ? 4 : 0)
+    k_sten(SolverArgs a, Coef<T> c, SolverBufs B, Red2 R, SolverScalars* S) {
     constexpr int NV = (OP == OP_SETUP || OP == OP_MATC) ? 2 : 1;
     constexpr bool RED = OP == OP_SETUP || OP == OP_MATC || OP == OP_MATP;
     __shared__ double smem[64];
@@ -550,10 +553,29 @@ __global__ void __launch_bounds__(256) k_sten(SolverArgs a, Coef<T> c, SolverBuf
     // other kernels the extra registers cost more occupancy than they save
     constexpr bool MARCH = OP == OP_SW1;
     const int ni = MARCH ? a.ni : 1;
-    if constexpr (!RED) {
+    if constexpr (!RED && !PS) {
         const int j = 1 + blockIdx.y * blockDim.y + threadIdx.y;
+        const int z = B.back ? gridDim.z - 1 - blockIdx.z : blockIdx.z;
         if (j <= d.jp)
-            sten_task<T, OP, MODE, NV, MARCH, V>(C, blockIdx.x, j, 1 + blockIdx.z * ni, ni, acc);
+            sten_task<T, OP, MODE, NV, MARCH, V>(C, blockIdx.x, j, 1 + z * ni, ni, acc);
+    } else if constexpr (!RED) {
+        const int lane = threadIdx.x & 31;
+        for (TaskIter t(blockIdx.x * blockDim.y + threadIdx.y, gridDim.x * blockDim.y, a.nkt,
+                        d.jp);
+             t.i <= d.ip; t.next()) {
+            TaskIter u = t;
+            u.next();
+            if (u.i <= d.ip) {  // the next task's lines
+                const int o = d.at(min(1 + V * (u.kt * BX + lane), d.kp), 1 + u.jr,
+                                   B.back ? d.ip + 1 - u.i : u.i);
+                prefetch_l2(C.gx + o);
+                prefetch_l2(C.rh + o);
+                prefetch_l2(C.vh + o);
+                if (OP == OP_SW3P) prefetch_l2((const T*)B.out + o);
+            }
+            sten_task<T, OP, MODE, NV, MARCH, V>(C, t.kt, 1 + t.jr,
+                                                 B.back ? d.ip + 1 - t.i : t.i, 1, acc);
+        }
     } else {
         const int lane = threadIdx.x & 31;
         // RM: a warp task is a column chunk over `rn` consecutive i-planes
@@ -1174,6 +1196,22 @@ static void sten_v(const SolverArgs& a, const Coef<T>& c, const SolverBufs& B, S
                    dim3(BX, BY), 0, st, a, c, B, w.red, w.S);
         }
     } else {
+        // FP64 sweeps two and three: persistent, with the next task's lines
+        // asked for ahead, once every resident warp has eight tasks or more.
+        // With the sweeps' alternating direction (launch_iteration) an
+        // iteration took 638 us before, 619 with the direction alone and 598
+        // with both at 256 x 256 x 128 (14 tasks a warp), 246 against 244 at
+        // 160 x 150 x 120 (10), and 84 against 88 at 128 x 96 x 64 (2.6, where the
+        // grid of one task a warp stays).  FP32 gained nothing.
+        if constexpr (std::is_same<T, double>::value && OP != OP_SW1) {
+            static const int full = persistent_grid(k_sten<T, OP, MODE, V, false, true>);
+            const long long tasks = (long long)a.nkt * a.d.jp * a.d.ip;
+            if (tasks >= 8LL * BY * full) {
+                launch(a.pdl, k_sten<T, OP, MODE, V, false, true>, dim3(full), dim3(BX, BY), 0, st,
+                       a, c, B, w.red, w.S);
+                return;
+            }
+        }
         // at most 256 threads: the kernels are compiled with __launch_bounds__(256)
         const int by = a.by >= 1 && a.by <= 256 / BX ? a.by : BY;
         const int ni = OP == OP_SW1 ? a.ni : 1;
@@ -1269,6 +1307,10 @@ static void launch_iteration(const SolverArgs& a, const Coef<T>& c, SolverWork<T
     B.rh = w.rh;
     B.vh = w.vh;
     const bool fused = fused_ok<T>(a);
+    // Separate sweeps alternate their direction along i, against the reducing
+    // kernels, whose order is fixed: a kernel then starts on the planes its
+    // predecessor touched last, which L2 still holds (a vector of 8 million
+    // FP64 points is 67 MB, a sweep touches four).
     SolverArgs a0 = a;  // the first kernel follows no kernel of this iteration
     a0.pdl = 0;
     // phase B: precondition(s <- t), p = s + bet p, v1 = A p
@@ -1280,14 +1322,17 @@ static void launch_iteration(const SolverArgs& a, const Coef<T>& c, SolverWork<T
     } else {
         B.out = w.sA;
         B.sweep = 1;
+        B.back = 1;
         sten<T, OP_SW1, 0>(a0, c, B, w, st, P_JACOBI);
         B.sin = w.sA;
         B.out = w.sB;
         B.sweep = 2;
+        B.back = 0;
         sten<T, OP_SW, 0>(a, c, B, w, st, P_JACOBI);
         B.sin = w.sB;
         B.out = w.p;
         B.sweep = 3;
+        B.back = 1;
         sten<T, OP_SW3P, 0>(a, c, B, w, st, P_JACOBI);
     }
     B.sin = w.p;
@@ -1307,14 +1352,17 @@ static void launch_iteration(const SolverArgs& a, const Coef<T>& c, SolverWork<T
     } else {
         B.out = w.sA;
         B.sweep = 1;
+        B.back = 1;
         sten<T, OP_SW1, 1>(a, c, B, w, st, P_JACOBI);
         B.sin = w.sA;
         B.out = w.sB;
         B.sweep = 2;
+        B.back = 0;
         sten<T, OP_SW, 1>(a, c, B, w, st, P_JACOBI);
         B.sin = w.sB;
         B.out = w.sA;
         B.sweep = 3;
+        B.back = 1;
         sten<T, OP_SW, 1>(a, c, B, w, st, P_JACOBI);
     }
     if (!mv) {
