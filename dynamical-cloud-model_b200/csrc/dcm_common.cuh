@@ -87,14 +87,6 @@ __device__ __forceinline__ double div_r(double a, double b, double r) {
 template <typename T>
 __device__ __forceinline__ T ld(const T* p) { return __ldg(p); }
 
-// a / b of the step's kernels.  FP64 (the parity path): the correctly rounded
-// divide.  FP32 (the mixed form): the two-instruction approximate divide,
-// within 2 ulp for divisors of magnitude 2^-126..2^126, which spacings,
-// densities and the limiter's sums (at least 1e-30) have; in that range it
-// returns the bits of the full-range sequence that -prec-div=false gives `/`.
-__device__ __forceinline__ double qdiv(double a, double b) { return a / b; }
-__device__ __forceinline__ float qdiv(float a, float b) { return __fdividef(a, b); }
-
 // periodic wrap of a halo index onto the interior 1..n
 __device__ __forceinline__ int wrapc(int c, int n) {
     return c < 1 ? c + n : (c > n ? c - n : c);

@@ -207,37 +207,37 @@ __global__ void __launch_bounds__(256) k_sources(Dims d, Metrics<T> mt, Forcing<
     const T rn = ld(mt.rhoan + k), ra = ld(mt.rhoa + k);
     const int o = d.at(k, j, i);
     // :746-754
-    T vsu = rn * ((qdiv(U(k, j, i - 1) * (U(k, j, i) + U(k, j, i - 1)) -
-                            U(k, j, i + 1) * (U(k, j, i) + U(k, j, i + 1)),
-                        two * (dx + dxm)) +
-                   qdiv(U(k, j - 1, i) * (V(k, j - 1, i) + V(k, j - 1, i + 1)) -
-                            U(k, j + 1, i) * (V(k, j, i) + V(k, j, i + 1)),
-                        two * (dyn + dynm)) +
-                   qdiv(U(k - 1, j, i) * (W(k - 1, j, i) + W(k - 1, j, i + 1)) -
-                            U(k + 1, j, i) * (W(k, j, i) + W(k, j, i + 1)),
-                        two * (dzn + dznm))));
+    T vsu = rn * (((U(k, j, i - 1) * (U(k, j, i) + U(k, j, i - 1)) -
+                    U(k, j, i + 1) * (U(k, j, i) + U(k, j, i + 1))) /
+                       (two * (dx + dxm)) +
+                   (U(k, j - 1, i) * (V(k, j - 1, i) + V(k, j - 1, i + 1)) -
+                    U(k, j + 1, i) * (V(k, j, i) + V(k, j, i + 1))) /
+                       (two * (dyn + dynm)) +
+                   (U(k - 1, j, i) * (W(k - 1, j, i) + W(k - 1, j, i + 1)) -
+                    U(k + 1, j, i) * (W(k, j, i) + W(k, j, i + 1))) /
+                       (two * (dzn + dznm))));
     // :765-773
-    T vsv = rn * ((qdiv(V(k, j, i - 1) * (U(k, j, i - 1) + U(k, j + 1, i - 1)) -
-                            V(k, j, i + 1) * (U(k, j, i) + U(k, j + 1, i)),
-                        two * (dxn + dxnm)) +
-                   qdiv(V(k, j - 1, i) * (V(k, j, i) + V(k, j - 1, i)) -
-                            V(k, j + 1, i) * (V(k, j, i) + V(k, j + 1, i)),
-                        two * (dy + dym)) +
-                   qdiv(V(k - 1, j, i) * (W(k - 1, j, i) + W(k - 1, j + 1, i)) -
-                            V(k + 1, j, i) * (W(k, j, i) + W(k, j + 1, i)),
-                        two * (dzn + dznm))));
+    T vsv = rn * (((V(k, j, i - 1) * (U(k, j, i - 1) + U(k, j + 1, i - 1)) -
+                    V(k, j, i + 1) * (U(k, j, i) + U(k, j + 1, i))) /
+                       (two * (dxn + dxnm)) +
+                   (V(k, j - 1, i) * (V(k, j, i) + V(k, j - 1, i)) -
+                    V(k, j + 1, i) * (V(k, j, i) + V(k, j + 1, i))) /
+                       (two * (dy + dym)) +
+                   (V(k - 1, j, i) * (W(k - 1, j, i) + W(k - 1, j + 1, i)) -
+                    V(k + 1, j, i) * (W(k, j, i) + W(k, j + 1, i))) /
+                       (two * (dzn + dznm))));
     // :784-794
-    T vsw = ra * ((qdiv(W(k, j, i - 1) * (U(k, j, i - 1) + U(k + 1, j, i - 1)) -
-                            W(k, j, i + 1) * (U(k, j, i) + U(k + 1, j, i)),
-                        two * (dxn + dxnm)) +
-                   qdiv(W(k, j - 1, i) * (V(k, j - 1, i) + V(k + 1, j - 1, i)) -
-                            W(k, j + 1, i) * (V(k, j, i) + V(k + 1, j, i)),
-                        two * (dyn + dynm)) +
-                   qdiv(W(k - 1, j, i) * (W(k, j, i) + W(k - 1, j, i)) -
-                            W(k + 1, j, i) * (W(k, j, i) + W(k + 1, j, i)),
-                        two * (dz + dzm))) +
-                  qdiv(T(9.81) * (th[o] + th[d.at(k + 1, j, i)]),
-                       two * ld(mt.theta + k) + ld(thbar + k) + ld(thbar + k + 1)));
+    T vsw = ra * (((W(k, j, i - 1) * (U(k, j, i - 1) + U(k + 1, j, i - 1)) -
+                    W(k, j, i + 1) * (U(k, j, i) + U(k + 1, j, i))) /
+                       (two * (dxn + dxnm)) +
+                   (W(k, j - 1, i) * (V(k, j - 1, i) + V(k + 1, j - 1, i)) -
+                    W(k, j + 1, i) * (V(k, j, i) + V(k + 1, j, i))) /
+                       (two * (dyn + dynm)) +
+                   (W(k - 1, j, i) * (W(k, j, i) + W(k - 1, j, i)) -
+                    W(k + 1, j, i) * (W(k, j, i) + W(k + 1, j, i))) /
+                       (two * (dz + dzm))) +
+                  T(9.81) * (th[o] + th[d.at(k + 1, j, i)]) /
+                      (two * ld(mt.theta + k) + ld(thbar + k) + ld(thbar + k + 1)));
     T vsth = sth_reset ? T(0) : sth[o];
     if (F.damping_layer) {
         vsu = vsu + rn * ld(F.dampfacn + k) * (zu[o] - ld(ubar + k));
@@ -408,9 +408,9 @@ __global__ void __launch_bounds__(256) k_momentum_step(Dims d, Metrics<T> mt, Me
     const T gx = (T)div_r(p[d.at(k, j, i + 1)] - pc, ld(mtp.dxn + i), ld(mtp.rdxn + i));
     const T gy = (T)div_r(p[d.at(k, j + 1, i)] - pc, ld(mtp.dyn + j), ld(mtp.rdyn + j));
     const T gz = (T)div_r(p[d.at(k + 1, j, i)] - pc, ld(mtp.dzn + k), ld(mtp.rdzn + k));
-    const T nu = zuo + qdiv((su[o] - gx) * dt2, ld(mt.rhoan + k));
-    const T nv = zvo + qdiv((sv[o] - gy) * dt2, ld(mt.rhoan + k));
-    const T nw = zwo + qdiv((sw[o] - gz) * dt2, ld(mt.rhoa + k));
+    const T nu = zuo + ((su[o] - gx) * dt2) / ld(mt.rhoan + k);
+    const T nv = zvo + ((sv[o] - gy) * dt2) / ld(mt.rhoan + k);
+    const T nw = zwo + ((sw[o] - gz) * dt2) / ld(mt.rhoa + k);
     put_plane_images(tu, d, k, j, i, nu);
     put_plane_images(tv, d, k, j, i, nv);
     put_plane_images(tw, d, k, j, i, nw);
@@ -453,12 +453,12 @@ __global__ void __launch_bounds__(256) k_adv_ref(Dims d, Metrics<T> mt, T dt,
     if (k > d.kp || j > (exch ? d.jp : d.jp + 1)) return;
     const int o = d.at(k, j, i);
     const T h = T(0.5);
-    const T v =
-        psi[o] - qdiv(dt * (qdiv(h, ld(mt.dz + k - 1)) * w[d.at(k - 1, j, i)] *
-                                ld(mt.rhoa + k - 1) * (ld(ref + k) - ld(ref + k - 1)) +
-                            qdiv(h, ld(mt.dz + k)) * w[o] * ld(mt.rhoa + k) *
-                                (ld(ref + k + 1) - ld(ref + k))),
-                      ld(mt.rhoan + k));
+    const T v = psi[o] - dt *
+                             (h / ld(mt.dz + k - 1) * w[d.at(k - 1, j, i)] * ld(mt.rhoa + k - 1) *
+                                  (ld(ref + k) - ld(ref + k - 1)) +
+                              h / ld(mt.dz + k) * w[o] * ld(mt.rhoa + k) *
+                                  (ld(ref + k + 1) - ld(ref + k))) /
+                             ld(mt.rhoan + k);
     if (exch)
         put_full(out, d, k, j, i, v, T(0), T(0));
     else

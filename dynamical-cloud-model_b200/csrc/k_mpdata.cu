@@ -96,14 +96,14 @@ __device__ __forceinline__ T donor_point(const Dims& d, const Metrics<T>& mt, T 
     const T pc = P(k, j, i);
     const T dxn = ld(mt.dxn + i), dyn = ld(mt.dyn + j), dzn = ld(mt.dzn + k);
     const T ra = ld(mt.rhoa + k), ram = ld(mt.rhoa + k - 1), rn = ld(mt.rhoan + k);
-    const T fxr = qdiv(((uc + fabs(uc)) * pc + (uc - fabs(uc)) * P(k, j, i + 1)) * dt, two * dxn);
-    const T fxl = qdiv(((um + fabs(um)) * P(k, j, i - 1) + (um - fabs(um)) * pc) * dt, two * dxn);
-    const T fyr = qdiv(((vc + fabs(vc)) * pc + (vc - fabs(vc)) * P(k, j + 1, i)) * dt, two * dyn);
-    const T fyl = qdiv(((vm + fabs(vm)) * P(k, j - 1, i) + (vm - fabs(vm)) * pc) * dt, two * dyn);
-    T fzr = qdiv(((wc + fabs(wc)) * ra * pc + (wc - fabs(wc)) * ra * P(k + 1, j, i)) * dt,
-                 two * dzn * rn);
-    T fzl = qdiv(((wm + fabs(wm)) * ram * P(k - 1, j, i) + (wm - fabs(wm)) * ram * pc) * dt,
-                 two * dzn * rn);
+    const T fxr = ((uc + fabs(uc)) * pc + (uc - fabs(uc)) * P(k, j, i + 1)) * dt / (two * dxn);
+    const T fxl = ((um + fabs(um)) * P(k, j, i - 1) + (um - fabs(um)) * pc) * dt / (two * dxn);
+    const T fyr = ((vc + fabs(vc)) * pc + (vc - fabs(vc)) * P(k, j + 1, i)) * dt / (two * dyn);
+    const T fyl = ((vm + fabs(vm)) * P(k, j - 1, i) + (vm - fabs(vm)) * pc) * dt / (two * dyn);
+    T fzr = ((wc + fabs(wc)) * ra * pc + (wc - fabs(wc)) * ra * P(k + 1, j, i)) * dt /
+            (two * dzn * rn);
+    T fzl = ((wm + fabs(wm)) * ram * P(k - 1, j, i) + (wm - fabs(wm)) * ram * pc) * dt /
+            (two * dzn * rn);
     if (neumann == 1) {  // :98-104
         if (k == 1) fzl = fzr;
         if (k == d.kp) fzr = fzl;
@@ -366,17 +366,19 @@ __device__ __forceinline__ void beta0_point(const Dims& d, const Metrics<T>& mt,
         pmin = fmin(pmin, s[q]);
     }
     const T denom1 =
-        dt * (qdiv(fmax(Uim, z) * rn * PO(k, j, i - 1) - fmin(Uc, z) * rn * PO(k, j, i + 1), dxn) +
-              qdiv(fmax(Vjm, z) * rn * PO(k, j - 1, i) - fmin(Vc, z) * rn * PO(k, j + 1, i), dyn) +
-              qdiv(fmax(Wkm, z) * ram * PO(k - 1, j, i) - fmin(Wc, z) * ra * PO(k + 1, j, i),
-                   dzn)) +
+        dt * ((fmax(Uim, z) * rn * PO(k, j, i - 1) - fmin(Uc, z) * rn * PO(k, j, i + 1)) /
+                  dxn +
+              (fmax(Vjm, z) * rn * PO(k, j - 1, i) - fmin(Vc, z) * rn * PO(k, j + 1, i)) /
+                  dyn +
+              (fmax(Wkm, z) * ram * PO(k - 1, j, i) - fmin(Wc, z) * ra * PO(k + 1, j, i)) /
+                  dzn) +
         small;
     const T denom2 =
-        dt * (qdiv(fmax(Uc, z) * rn * pc - fmin(Uim, z) * rn * pc, dxn) +
-              qdiv(fmax(Vc, z) * rn * pc - fmin(Vjm, z) * rn * pc, dyn) +
-              qdiv(fmax(Wc, z) * ra * pc - fmin(Wkm, z) * ram * pc, dzn) + small);
-    bup = qdiv(rn * (pmax - pc), denom1);
-    bdn = qdiv(rn * (pc - pmin), denom2);
+        dt * ((fmax(Uc, z) * rn * pc - fmin(Uim, z) * rn * pc) / dxn +
+              (fmax(Vc, z) * rn * pc - fmin(Vjm, z) * rn * pc) / dyn +
+              (fmax(Wc, z) * ra * pc - fmin(Wkm, z) * ram * pc) / dzn + small);
+    bup = rn * (pmax - pc) / denom1;
+    bdn = rn * (pc - pmin) / denom2;
 }
 
 // one limited velocity component (eq 18, :634-656): c the antidiffusive
