@@ -150,7 +150,7 @@ struct SolverWork {
     int round_budget = 0;
     double tiny = -1.0;
     // FP64: domains of at most this many interior points solve in one
-    // thread-block cluster (k_bicgstab_small); 0 = never
+    // thread-block cluster (k_bicgstab_point, k_bicgstab_small); 0 = never
     long long small_max = 0;
     // mixed form: direct corrections ahead of the iterations (null or !ok: none)
     const DirectPlan* direct = nullptr;

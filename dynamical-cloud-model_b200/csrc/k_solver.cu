@@ -1072,7 +1072,8 @@ __global__ void __launch_bounds__(256) k_bicg_update(SolverArgs a, Coef<T> c,
 //     exchange_along_dim_wo(p) (driver_code.f90:506)
 // One thread per cell of the six faces of the interior (blockIdx.y: i, j, k
 // pair), which are all that have images; a cell on two faces is written twice
-// with the same values.
+// with the same values.  (A thread per interior point took 41 us at
+// 256 x 256 x 128, the faces take 11.)
 template <typename T, typename TS>
 __global__ void __launch_bounds__(256) k_bicg_post(Dims d, T* __restrict__ x,
                                                    const TS* __restrict__ sw,
