@@ -9,8 +9,8 @@ of the run from the initial state (a warm-up run of W steps precedes them on
 the same handle, then the initial state is uploaded again), so every arm
 times the same time steps with the same solver iteration counts.
 
-The headline `value` is the mixed-precision form (FP32 fields and BiCGSTAB
-iterations, FP64 pressure, residual and dot products); the plain FP64 path
+The headline `value` is the mixed-precision form (FP32 fields and pressure
+corrections, FP64 pressure, residual and dot products); the plain FP64 path
 is timed on the same steps (`fp64`), and the per-field max / RMS errors of
 the mixed form against the FP64 path after 1, 10 and --accuracy-steps steps
 go in `accuracy_vs_fp64`.
