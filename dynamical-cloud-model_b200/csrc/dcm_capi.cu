@@ -1057,6 +1057,13 @@ SolverWork<float> solver_work_f(dcm_handle* h) {
     w.cheb_lo = h->cfg.precond_lo > 0.0 ? h->cfg.precond_lo : 0.05;
     w.round_budget = h->round_budget;
     w.direct = &h->direct;
+    if (h->direct.keep) {  // the pressure at the start; without it the iterations alone
+        w.x_keep = slot(h, S_X);
+        if (!w.x_keep) {
+            cudaGetLastError();
+            w.direct = nullptr;
+        }
+    }
     return w;
 }
 

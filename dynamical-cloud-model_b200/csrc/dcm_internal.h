@@ -59,6 +59,18 @@ constexpr long long DIRECT_MAX_POINTS = 1 << 24;
 // a correction is followed by another while it lowers the residual by this
 // factor (one lowers it by about 1e-4); else the iterations take over
 constexpr double DIRECT_CONTRACTION = 0.25;
+// A correction is rounded to FP32, so it leaves a residual of about 2^-24 kappa
+// times the one it removes, kappa the ratio of the operator's largest
+// eigenvalue to its smallest but zero (of the horizontal modes; the mean mode
+// is solved in FP64 and counts against the vertical coefficients alone).
+// Measured on residuals of the lowest mode alone, the worst there are, for
+// kappa 3e3 to 2e9: 0.2 to 1.06 times that.  Beyond DIRECT_SURE a correction
+// may not contract, and the FP32 iterations do not get on from the pressure it
+// leaves (9 of 2^-24 kappa, 256 x 64 x 40 cells 3000 x 3000 x 20 m: they
+// stalled at 6e-9 and diverged), so the pressure is kept and put back for them.
+// Up to DIRECT_MOST warm bubbles on cells of dx/dz or dx/dy 1 to 300 converged
+// by corrections alone, in at most 11; above, most did not.
+constexpr double DIRECT_SURE = 0.2, DIRECT_MOST = 4.0;
 constexpr int DIRECT_MAX_RADICES = 12;
 constexpr size_t DIRECT_MAX_SMEM = 227 * 1024;  // of one transform block
 
@@ -71,6 +83,7 @@ struct DirectPlan {
     bool ok = false;
     AxisPlan axis[2];  // x, y
     const double *w = nullptr, *g = nullptr, *l = nullptr;  // mean mode (k_zsolve)
+    bool keep = false;  // the pressure is kept for the iterations (DIRECT_SURE)
     void* block = nullptr;  // the device tables
 };
 
@@ -154,6 +167,7 @@ struct SolverWork {
     long long small_max = 0;
     // mixed form: direct corrections ahead of the iterations (null or !ok: none)
     const DirectPlan* direct = nullptr;
+    double* x_keep = nullptr;  // FP64 field for the starting pressure (direct->keep)
 };
 
 // direct corrections (k_direct.cu)
@@ -167,11 +181,13 @@ int direct_plan_build(const Dims& d, const std::vector<double>& ae, const std::v
 void direct_correction(const DirectPlan& P, const Dims& d, const Coef<float>& c, const float* r,
                        float* work, double* x, cudaStream_t st);
 // r = b - A x and the loop's decision into S->direct, S->done, S->status (and
-// the WHILE node's condition)
+// the WHILE node's condition); first: x also goes to keep, unless null
 void direct_residual(const Dims& d, const Coef<double>& c, const double* x, const double* b,
-                     float* r, double tol, int itmax, int max_rounds, bool first, const Red2& red,
+                     double* keep, float* r, double tol, int itmax, int max_rounds, bool first, const Red2& red,
                      int max_blocks, SolverScalars* S, const cudaGraphConditionalHandle* cond,
                      cudaStream_t st);
+// x = keep (interior)
+void direct_put_back(const Dims& d, const double* keep, double* x, cudaStream_t st);
 
 // one-time setup of the solver kernels (shared-memory limits, the probe of
 // programmatic launches in graphs); called at handle creation, outside any

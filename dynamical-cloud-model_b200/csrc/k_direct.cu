@@ -11,7 +11,8 @@
 // or three corrections reach the 1e-10 that FP32 BiCGSTAB iterations need
 // 70 to 190 for (256 x 256 x 128 warm bubble).  refine_run (k_solver.cu)
 // takes the corrections and, where one does not contract the residual, goes
-// on with the BiCGSTAB iterations from there.
+// on with the BiCGSTAB iterations: from the pressure as corrected, or on
+// grids where that may be no better (DIRECT_SURE) from the one it started with.
 //
 // Kernels per correction, each one pass in and one pass out of one FP32 field:
 //   k_fft      transform along y (r -> scratch)
@@ -573,24 +574,33 @@ __global__ void __launch_bounds__(256) k_zsolve(ZArgs a, float* __restrict__ f) 
             zstore<V>(p, nmem, D);
             continue;
         }
-        const float lam = ld(a.lx + mx) + ld(a.ly + my);
-        float A[V], C[V];
-        // rows beyond kp: u = 0
+        const float lam = -(ld(a.lx + mx) + ld(a.ly + my));
+        // normalised rows u + A u(below) + C u(above) = D with A, C <= 0, and
+        // S = 1 + A + C, the row's excess over its neighbours (lam / diagonal
+        // at first), carried through the elimination: every diagonal is then a
+        // sum of positive terms.  Formed as 1 - products it loses the excess
+        // where lam is below the round-off of au + ad (flat cells: dx 50 dz and
+        // 512 points made the first mode's system singular).
+        float A[V], C[V], S[V];
 #pragma unroll
         for (int e = 0; e < V; e++) {
-            const float b = e < nvalid ? lam - ad[e] - au[e] : 1.0f;
+            // rows beyond kp: u = 0
+            float ex = e < nvalid ? lam : 1.0f;
             if (e < 2) {
-                const float r = __fdividef(1.0f, b);
+                const float r = __fdividef(-1.0f, ex + ad[e] + au[e]);
                 D[e] *= r;
                 E[e] *= r;
                 A[e] = ad[e] * r;
                 C[e] = au[e] * r;
+                S[e] = -r * ex;
             } else {
-                const float r = __fdividef(1.0f, b - ad[e] * C[e - 1]);
+                ex += ad[e] * S[e - 1];
+                const float r = __fdividef(-1.0f, ex - ad[e] * A[e - 1] + au[e]);
                 D[e] = r * (D[e] - ad[e] * D[e - 1]);
                 E[e] = r * (E[e] - ad[e] * E[e - 1]);
                 A[e] = -r * ad[e] * A[e - 1];
                 C[e] = r * au[e];
+                S[e] = -r * ex;
             }
         }
 #pragma unroll
@@ -598,36 +608,42 @@ __global__ void __launch_bounds__(256) k_zsolve(ZArgs a, float* __restrict__ f) 
             D[e] -= C[e] * D[e + 1];
             E[e] -= C[e] * E[e + 1];
             A[e] -= C[e] * A[e + 1];
+            S[e] -= C[e] * S[e + 1];
             C[e] = -C[e] * C[e + 1];
         }
         if (V > 2) {
-            const float r = __fdividef(1.0f, 1.0f - C[0] * A[1]);
+            const float ex = S[0] - C[0] * S[1];
+            const float r = __fdividef(1.0f, ex - A[0] + C[0] * C[1]);
             D[0] = r * (D[0] - C[0] * D[1]);
             E[0] = r * (E[0] - C[0] * E[1]);
             A[0] = r * A[0];
             C[0] = -r * C[0] * C[1];
+            S[0] = r * ex;
         }
         // the last levels: first levels of this lane and the next eliminated
         const float dn = __shfl_down_sync(FULL, D[0], 1), en = __shfl_down_sync(FULL, E[0], 1),
-                    an = __shfl_down_sync(FULL, A[0], 1), cn = __shfl_down_sync(FULL, C[0], 1);
+                    sn = __shfl_down_sync(FULL, S[0], 1), cn = __shfl_down_sync(FULL, C[0], 1);
         const float al = A[V - 1], cl = C[V - 1];
-        float r = __fdividef(1.0f, 1.0f - al * C[0] - cl * an);
+        float ex = S[V - 1] - al * S[0] - cl * sn;
+        float r = __fdividef(1.0f, ex + al * A[0] + cl * cn);
         float x = r * (D[V - 1] - al * D[0] - cl * dn);
         float y = r * (E[V - 1] - al * E[0] - cl * en);
-        float lo = -r * al * A[0], up = -r * cl * cn;
+        float lo = -r * al * A[0], up = -r * cl * cn, sx = r * ex;
 #pragma unroll
         for (int s = 1; s < 32; s <<= 1) {
             // lo is 0 in the first s lanes and up in the last s, so what the
             // shuffles return there does not count
             const float xm = __shfl_up_sync(FULL, x, s), ym = __shfl_up_sync(FULL, y, s),
-                        lm = __shfl_up_sync(FULL, lo, s), um = __shfl_up_sync(FULL, up, s);
+                        lm = __shfl_up_sync(FULL, lo, s), sm = __shfl_up_sync(FULL, sx, s);
             const float xp = __shfl_down_sync(FULL, x, s), yp = __shfl_down_sync(FULL, y, s),
-                        lp = __shfl_down_sync(FULL, lo, s), upp = __shfl_down_sync(FULL, up, s);
-            r = __fdividef(1.0f, 1.0f - lo * um - up * lp);
+                        sp = __shfl_down_sync(FULL, sx, s), upp = __shfl_down_sync(FULL, up, s);
+            ex = sx - lo * sm - up * sp;
+            r = __fdividef(1.0f, ex + lo * lm + up * upp);
             x = r * (x - lo * xm - up * xp);
             y = r * (y - lo * ym - up * yp);
             lo = -r * lo * lm;
             up = -r * up * upp;
+            sx = r * ex;
         }
         float px1 = __shfl_up_sync(FULL, x, 1), py1 = __shfl_up_sync(FULL, y, 1);
         if (lane == 0) px1 = py1 = 0.0f;
@@ -666,6 +682,7 @@ struct DirResidualArgs {
     Dims d;
     Coef<double> c;
     const double *x, *b;
+    double* keep;  // FIRST: a copy of x, unless null
     float* r;
     double tol;
     int itmax, max_rounds;
@@ -714,6 +731,13 @@ __global__ void __launch_bounds__(256, 4) k_dir_residual(DirResidualArgs a, Red2
                                       au0 * up0 + (sij - au0 - ad0) * xc.x);
             const double r1 = bv.y - (aw * xw.y + ae * xe.y + as * xs.y + an * xn.y + ad1 * xc.x +
                                       au1 * next + (sij - au1 - ad1) * xc.y);
+            if (FIRST && a.keep && live) {
+                double* kx = a.keep + kl + d.K * j + o;
+                if (both)
+                    *reinterpret_cast<double2*>(kx) = xc;
+                else
+                    *kx = xc.x;
+            }
             if (live) {
                 acc[0] += r0 * r0;
                 if (FIRST) acc[1] += bv.x * bv.x;
@@ -780,6 +804,15 @@ __global__ void __launch_bounds__(256, 4) k_dir_residual(DirResidualArgs a, Red2
     if (a.use_cond) cudaGraphSetConditional(a.cond, (unsigned)go);
 }
 
+__global__ void __launch_bounds__(256) k_dir_put_back(Dims d, const double* __restrict__ keep,
+                                                      double* __restrict__ x) {
+    const int k = 1 + blockIdx.x * BX + threadIdx.x;
+    const int j = 1 + blockIdx.y * BY + threadIdx.y;
+    const int i = 1 + blockIdx.z;
+    if (k > d.kp || j > d.jp) return;
+    x[d.at(k, j, i)] = keep[d.at(k, j, i)];
+}
+
 // ---- host side ----------------------------------------------------------------------
 namespace {
 
@@ -827,6 +860,25 @@ bool uniform(const std::vector<double>& a, const std::vector<double>& b, int n) 
     return a[1] > 0.0;
 }
 
+// ratio of the largest eigenvalue to the smallest of the horizontal modes, or
+// of the mean mode's vertical coefficients (its smallest from the column's
+// height in units of the local spacing: (pi / sum of 1 / sqrt(a))^2)
+double condition(const Dims& d, double ax, double ay, const std::vector<double>& au,
+                 const std::vector<double>& ad) {
+    double v = 0.0, height = 0.0;
+    for (int k = 1; k <= d.kp; k++) {
+        v = std::max(v, 2.0 * (au[k] + ad[k]));
+        height += 1.0 / std::sqrt(std::sqrt(au[k] * ad[k]));
+    }
+    const double pi = 0.5 * kTwoPi;
+    const double sx = std::sin(pi / d.ip), sy = std::sin(pi / d.jp);
+    double low = HUGE_VAL;
+    if (d.ip > 1) low = std::min(low, 4.0 * ax * sx * sx);
+    if (d.jp > 1) low = std::min(low, 4.0 * ay * sy * sy);
+    const double top = (d.ip > 1 ? 4.0 * ax : 0.0) + (d.jp > 1 ? 4.0 * ay : 0.0) + v;
+    return std::max(top / low, v * (height / pi) * (height / pi));
+}
+
 // sequences per tile: 16 (128-byte segments) while two buffers of a line
 // leave room for three blocks per SM, else 8
 int tile_pairs(int n) { return n <= 288 ? 16 : 8; }
@@ -858,6 +910,9 @@ int direct_plan_build(const Dims& d, const std::vector<double>& ae, const std::v
     }
     for (int k = 1; k <= d.kp; k++)
         if (!(au[k] > 0.0 && ad[k] > 0.0)) return DCM_OK;
+    const double noise = std::ldexp(condition(d, ae[1], an[1], au, ad), -24);
+    if (!(noise <= DIRECT_MOST)) return DCM_OK;
+    P.keep = noise > DIRECT_SURE;
     // one block: per axis n roots (float2) and n eigenvalues, then the mean
     // mode's tables (kp + 2 doubles each)
     std::vector<float> f;
@@ -984,8 +1039,13 @@ void direct_correction(const DirectPlan& P, const Dims& d, const Coef<float>& c,
     fft(P, d, 1, FFT_ADD, work, nullptr, x, st);
 }
 
+void direct_put_back(const Dims& d, const double* keep, double* x, cudaStream_t st) {
+    ProfScope ps(P_OTHER, st);
+    k_dir_put_back<<<interior_grid(d, d.kp), dim3(BX, BY), 0, st>>>(d, keep, x);
+}
+
 void direct_residual(const Dims& d, const Coef<double>& c, const double* x, const double* b,
-                     float* r, double tol, int itmax, int max_rounds, bool first, const Red2& red,
+                     double* keep, float* r, double tol, int itmax, int max_rounds, bool first, const Red2& red,
                      int max_blocks, SolverScalars* S, const cudaGraphConditionalHandle* cond,
                      cudaStream_t st) {
     DirResidualArgs a;
@@ -993,6 +1053,7 @@ void direct_residual(const Dims& d, const Coef<double>& c, const double* x, cons
     a.c = c;
     a.x = x;
     a.b = b;
+    a.keep = first ? keep : nullptr;
     a.r = r;
     a.tol = tol;
     a.itmax = itmax;

@@ -2529,13 +2529,14 @@ int refine_run(SolverWork<float>& wf, SolverWork<double>& wd, const Dims& d, dou
     const int g = red_grid(a, gfull, a.nkt, a.ni);
     const dim3 gi = interior_grid(d, d.kp), bl(BX, BY);
     const bool direct = wf.direct && wf.direct->ok;
+    double* const keep = direct && wf.direct->keep ? wf.x_keep : nullptr;
     a.after_direct = direct ? 1 : 0;
     const int max_rounds = wf.round_budget > 0 ? wf.round_budget : itmax + max_updates + 1;
     auto start = [&](cudaStream_t s) { k_ru_begin<<<1, 1, 0, s>>>(wf.S, delta); };
     // the residual of a direct phase; the correction it calls for
     auto dir_residual = [&](cudaStream_t s, bool first, const cudaGraphConditionalHandle* h) {
-        direct_residual(d, cd, x, b, wf.r, tol, itmax, max_rounds, first, wd.red, wf.max_blocks,
-                        wf.S, h, s);
+        direct_residual(d, cd, x, b, keep, wf.r, tol, itmax, max_rounds, first, wd.red,
+                        wf.max_blocks, wf.S, h, s);
     };
     auto dir_correct = [&](cudaStream_t s) {
         direct_correction(*wf.direct, d, cf, wf.r, wf.sA, x, s);
@@ -2629,6 +2630,7 @@ int refine_run(SolverWork<float>& wf, SolverWork<double>& wd, const Dims& d, dou
             if (good) k_branch_iterate<<<1, 1, 0, s0>>>(hk, wf.S);
             good = good && capture_cond_node(s0, hk, cudaGraphCondTypeIf, 1, rest);
             good = good && capture_into(G.side[0], rest[0], [&](cudaStream_t s) {
+                       if (keep) direct_put_back(d, keep, x, s);
                        if (!emit_iterations(s, G, 1)) good = false;
                    });
         }
@@ -2643,7 +2645,7 @@ int refine_run(SolverWork<float>& wf, SolverWork<double>& wd, const Dims& d, dou
         const double kd[3] = {tol, delta, af.cheb ? wf.cheb_lo : 0.0};
         const int shape = af.by + 16 * af.tasks + 256 * af.ni + 16384 * af.fuse +
                           65536 * af.cheb + 131072 * (wf.pdl ? 1 : 0) + 262144 * af.vw +
-                          2097152 * (direct ? 1 : 0);
+                          2097152 * (direct ? 1 : 0);  // keep: with the grid
         const int ki[6] = {itmax, max_updates, 1 + 2 * max_rounds, 16 * shape,
                            d.ip * 4096 + d.jp, d.kp};
         if (!G.matches(kp, kd, ki)) {
@@ -2680,6 +2682,7 @@ int refine_run(SolverWork<float>& wf, SolverWork<double>& wd, const Dims& d, dou
             }
             iterate = !hS_in->done;
         }
+        if (iterate && keep) direct_put_back(d, keep, x, st);
         if (iterate) begin(st);
         int launched = 0;
         for (int round = 0; iterate; round++) {
@@ -2717,7 +2720,7 @@ int refine_run(SolverWork<float>& wf, SolverWork<double>& wd, const Dims& d, dou
             g_prof->add(P_JACOBI, (fused_ok<float>(af) ? 2 : 6) * itr);
             g_prof->add(P_MATVEC, (fused_ok<float>(af) && af.fuse_mv ? 1 : 2) * itr);
             g_prof->add(P_UPDATE, itr + u + 1);
-            g_prof->add(P_OTHER, 3 * cyc + 1);
+            g_prof->add(P_OTHER, 3 * cyc + 1 + (keep ? 1 : 0));
         }
         g_prof->add(P_POST, 1);
         g_prof->add(P_OTHER, direct ? 3 : 2);

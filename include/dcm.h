@@ -237,7 +237,11 @@ typedef struct {
                                lowered by direct corrections, FP32 solves of
                                A dx = r by transforms in x and y and
                                tridiagonal systems in z; the iterations
-                               follow where one does not contract it       */
+                               follow where one does not contract it.
+                               Grids whose operator FP32 cannot resolve
+                               (about ip dx > 25000 dz or dy, or the same
+                               of jp dy: very flat or oblong ones) take the
+                               iterations alone                            */
     double inner_tol;       /* precision 1: reliable-update factor: the FP32
                                recursion stops for an FP64 update of p and
                                of the true residual when its residual has

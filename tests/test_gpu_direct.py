@@ -101,3 +101,72 @@ def test_limits_of_the_direct_corrections(dcm):
         assert core.step(1).err_last < c.ptol
     finally:
         core.close()
+
+
+def _flat(shape, dx, dy, dz, mode=None, amp=0.0):
+    """A bubble and noise on cells of dx, dy, dz, at rest; with mode, the
+    starting pressure holds amp times that axis' longest wave."""
+    ip, jp, kp = shape
+    g = cases.make_grid(ip, jp, kp, dx, dy, dz, [-1.0e4, 1.0e5], [300.0, 300.0])
+    rng = np.random.default_rng(65)
+    r = np.sqrt((g.xn[None, None, 1:-1] / (0.2 * ip * dx)) ** 2 +
+                (g.yn[None, 1:-1, None] / (0.2 * jp * dy)) ** 2 +
+                ((g.zn[1:-1, None, None] - 0.5 * kp * dz) / (0.25 * kp * dz)) ** 2)
+    th, p = cases.fzeros(kp, jp, ip), cases.fzeros(kp, jp, ip)
+    th[1:-1, 1:-1, 1:-1] = 2.0 * np.cos(0.5 * np.pi * np.minimum(r, 1.0)) ** 2 + \
+        rng.normal(0.0, 0.01, size=(kp, jp, ip))
+    cases.exchange_full(th)
+    if mode == "x":
+        p[1:-1, 1:-1, 1:-1] = amp * np.cos(2 * np.pi * np.arange(ip) / ip)[None, None, :]
+    st = cases.State(*(cases.fzeros(kp, jp, ip) for _ in range(9)), th, p)
+    return g, st
+
+
+# flat and oblong cells: 2^-24 times the operator's condition from 0.01 to 400
+@pytest.mark.parametrize("shape,d", [
+    ((256, 64, 40), (200.0, 200.0, 20.0)), ((256, 64, 40), (1000.0, 1000.0, 20.0)),
+    ((256, 64, 40), (2000.0, 2000.0, 20.0)), ((256, 64, 40), (3000.0, 3000.0, 20.0)),
+    ((256, 64, 40), (20000.0, 20000.0, 20.0)), ((97, 40, 70), (1000.0, 1000.0, 20.0)),
+    ((64, 64, 130), (900.0, 900.0, 20.0)), ((64, 64, 300), (1500.0, 1500.0, 20.0)),
+    ((256, 64, 40), (6000.0, 20.0, 20.0)), ((64, 256, 40), (20.0, 2000.0, 20.0)),
+    ((3, 1500, 40), (20.0, 1000.0, 20.0))])
+def test_flat_cells(dcm, shape, d):
+    """Every solve converges, to the FP64 path's pressure within the mixed
+    form's bar."""
+    g, state = _flat(shape, *d)
+    out = []
+    for precision in (1, 0):
+        core = dcm.DynamicalCore(g)
+        core.upload_state(state, 1.0, ptol=1e-10, kord=3, precision=precision)
+        core.driver_start()
+        for _ in range(2):
+            assert core.step(1).err_last < 1e-10
+        out.append(core.download_state())
+        core.close()
+    p32, p64 = (f["p"][1:-1, 1:-1, 1:-1] for f in out)
+    assert relerr(p32 - p32.mean(), p64 - p64.mean()) <= 1e-6
+
+
+def test_pressure_is_put_back_for_the_iterations(dcm):
+    """A correction that does not contract (flat cells, a starting pressure
+    whose residual is the longest wave's) is undone: a round budget of that one
+    correction ends the solve with the pressure it started with, and the
+    iterations that follow are the same from a graph and from the host."""
+    g, state = _flat((256, 64, 40), 1400.0, 1400.0, 20.0, "x", 1e5)
+    out = []
+    for graphs, itmax, rounds, status in ((1, 9999, 1, dcm.DCM_E_TIMEOUT),
+                                          (1, 10, 0, dcm.DCM_E_NOCONV),
+                                          (0, 10, 0, dcm.DCM_E_NOCONV)):
+        core = dcm.DynamicalCore(g)
+        core.solver_graphs(graphs)
+        core.upload_state(state, 1.0, ptol=1e-10, kord=3, precision=1, itmax=itmax)
+        core.driver_start()
+        core.solver_limits(max_rounds=rounds)
+        with pytest.raises(dcm.DCMError) as e:
+            core.step(1)
+        assert e.value.status == status
+        out.append(core.download_state()["p"][1:-1, 1:-1, 1:-1])
+        core.close()
+    start = state.p[1:-1, 1:-1, 1:-1]
+    assert np.array_equal(out[0], start)
+    assert np.array_equal(out[1], out[2]) and not np.array_equal(out[1], start)
