@@ -43,22 +43,26 @@ def up_to_date():
     return all(os.path.getmtime(p) <= t for p in deps())
 
 
-def build(force=False, verbose=False, extra=()):
-    if not force and up_to_date():
-        return LIB
+def objects(force=False, verbose=False, extra=()):
+    """The objects of all sources, compiling those older than their source or
+    any header."""
     objdir = os.path.join(HERE, "_build")
     os.makedirs(objdir, exist_ok=True)
+    shared = max(os.path.getmtime(p) for p in deps() if not p.endswith(".cu"))
     objs = []
     procs = []
     for src in sources():
         obj = os.path.join(objdir, os.path.basename(src) + ".o")
+        objs.append(obj)
+        if not force and os.path.exists(obj) and \
+                os.path.getmtime(obj) >= max(shared, os.path.getmtime(src)):
+            continue
         cmd = [NVCC] + ARCH + FLAGS + FILE_FLAGS.get(os.path.basename(src), []) + \
             list(extra) + ["-c", src, "-o", obj]
         if verbose:
             print(" ".join(cmd), flush=True)
         procs.append((src, subprocess.Popen(cmd, stdout=subprocess.PIPE,
                                             stderr=subprocess.STDOUT)))
-        objs.append(obj)
     failed = []
     for src, p in procs:
         out, _ = p.communicate()
@@ -71,6 +75,13 @@ def build(force=False, verbose=False, extra=()):
         for src, text in failed:
             sys.stderr.write(f"nvcc failed on {src}:\n{text}\n")
         raise RuntimeError("CUDA build failed")
+    return objs
+
+
+def build(force=False, verbose=False, extra=()):
+    if not force and up_to_date():
+        return LIB
+    objs = objects(force, verbose, extra)
     tmp = LIB + ".tmp"
     cmd = [NVCC] + ARCH + ["-shared", "-cudart", "static", "-o", tmp] + objs
     if verbose:

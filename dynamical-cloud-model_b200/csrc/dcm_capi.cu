@@ -112,6 +112,7 @@ struct dcm_handle {
     // dcm_set_small_solver: FP64 solves of at most this many interior points
     // run as one thread-block cluster
     long long small_max = 8192;
+    int small_blocks = 8;  // of this handle's device
     // dcm_set_mpdata_shape: fused antidiffusive iterations (off by default:
     // slower on B200, see dcm.h), their row cap
     int mp_fuse = 0, mp_rows = 32;
@@ -277,6 +278,7 @@ SolverWork<double> solver_work(dcm_handle* h) {
     w.round_budget = h->round_budget;
     w.tiny = h->tiny;
     w.small_max = h->small_max;
+    w.small_blocks = h->small_blocks;
     return w;
 }
 
@@ -402,7 +404,7 @@ extern "C" int dcm_create(const dcm_grid* g, int device, dcm_handle** out) {
     h->nh = h->hd.n();
     CK(cudaSetDevice(device));
     CK(cudaStreamCreateWithFlags(&h->st, cudaStreamNonBlocking));
-    solver_init();
+    h->small_blocks = solver_init();
     mpdata_init();
     direct_init();
     CK(cudaEventCreate(&h->ev0));

@@ -165,6 +165,7 @@ struct SolverWork {
     // FP64: domains of at most this many interior points solve in one
     // thread-block cluster (k_bicgstab_point, k_bicgstab_small); 0 = never
     long long small_max = 0;
+    int small_blocks = 8;  // blocks of that cluster (solver_init)
     // mixed form: direct corrections ahead of the iterations (null or !ok: none)
     const DirectPlan* direct = nullptr;
     double* x_keep = nullptr;  // FP64 field for the starting pressure (direct->keep)
@@ -192,7 +193,9 @@ void direct_put_back(const Dims& d, const double* keep, double* x, cudaStream_t 
 // one-time setup of the solver kernels (shared-memory limits, the probe of
 // programmatic launches in graphs); called at handle creation, outside any
 // stream capture
-void solver_init();
+// the blocks of the small solve's cluster on the current device: 16 where it can
+// place that many, else 8
+int solver_init();
 // whether graph-driven iterations can use programmatic dependent launch
 bool solver_pdl_available();
 

@@ -1273,13 +1273,10 @@ static void precond3(const SolverArgs& a, const Coef<float>& c, const SolverBufs
 
 // programmatic edges inside the graph-driven iterations (probed once)
 static int g_pdl_graphs = 0;
-// clusters of 16 blocks for the small solve (asked once: they need an SM group
-// with 16 free SMs)
-static int g_cluster16 = 0;
-static bool probe_cluster16();
+static int small_cluster();
 static bool probe_pdl_graphs();
 
-void solver_init() {
+int solver_init() {
     const int sm0 = (int)precond3_smem<0, false>(), sm1 = (int)precond3_smem<1, false>(),
               sm1m = (int)precond3_smem<1, true>();
     cudaFuncSetAttribute(k_precond3<0, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm0);
@@ -1291,10 +1288,8 @@ void solver_init() {
     cudaFuncSetAttribute(k_precond3<1, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          sm1m);
     static std::once_flag probed;  // handles may be created from several threads
-    std::call_once(probed, [] {
-        g_pdl_graphs = probe_pdl_graphs() ? 1 : 0;
-        g_cluster16 = probe_cluster16() ? 1 : 0;
-    });
+    std::call_once(probed, [] { g_pdl_graphs = probe_pdl_graphs() ? 1 : 0; });
+    return small_cluster();
 }
 
 bool solver_pdl_available() { return g_pdl_graphs != 0; }
@@ -2078,7 +2073,10 @@ __global__ void __launch_bounds__(NT, 1)
     cl.sync();  // no block leaves while another may still read its operand
 }
 
-static bool probe_cluster16() {
+// The blocks of the small solve's cluster on the current device: 16 where it
+// has an SM group that can place one (the attribute, as every kernel's, is the
+// device's own), else the portable 8.
+static int small_cluster() {
     auto kern = k_bicgstab_point<512, 16>;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeClusterDimension;
@@ -2094,8 +2092,8 @@ static bool probe_cluster16() {
     const bool good =
         ok(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1)) &&
         ok(cudaOccupancyMaxActiveClusters(&clusters, kern, &cfg)) && clusters > 0;
-    cudaGetLastError();
-    return good;
+    if (!good) cudaGetLastError();
+    return good ? 16 : SMALL_CL;
 }
 
 // the one-cluster solve applies (FP64, interior points <= w.small_max)
@@ -2159,21 +2157,21 @@ int solver_run(SolverWork<T>& w, const Dims& d, T* x, const T* b, const T* sw, c
                 cfg.attrs = at;
                 cfg.numAttrs = 1;
                 // one point per thread where the cluster has as many
-                if (d.ip * d.jp * d.kp <= SMALL_CL * SMALL_THREADS) {
-                    if (g_cluster16) {
-                        at[0].val.clusterDim.x = 16;
-                        cfg.gridDim = dim3(16);
-                        cfg.blockDim = dim3(512);
-                        cudaLaunchKernelEx(&cfg, k_bicgstab_point<512, 16>, a, op, x, b, w.S,
+                cudaError_t e = cudaSuccess;
+                if (d.ip * d.jp * d.kp > SMALL_CL * SMALL_THREADS) {
+                    e = cudaLaunchKernelEx(&cfg, k_bicgstab_small, a, op, x, b, w.r, w.cr, w.p,
+                                           w.v1, w.t, w.sA, w.sB, w.rh, w.S, max_rounds);
+                } else if (w.small_blocks == 16) {
+                    at[0].val.clusterDim.x = 16;
+                    cfg.gridDim = dim3(16);
+                    cfg.blockDim = dim3(512);
+                    e = cudaLaunchKernelEx(&cfg, k_bicgstab_point<512, 16>, a, op, x, b, w.S,
                                            max_rounds);
-                    } else {
-                        cudaLaunchKernelEx(&cfg, k_bicgstab_point<SMALL_THREADS, SMALL_CL>, a, op,
+                } else {
+                    e = cudaLaunchKernelEx(&cfg, k_bicgstab_point<SMALL_THREADS, SMALL_CL>, a, op,
                                            x, b, w.S, max_rounds);
-                    }
                 }
-                else
-                    cudaLaunchKernelEx(&cfg, k_bicgstab_small, a, op, x, b, w.r, w.cr, w.p, w.v1,
-                                       w.t, w.sA, w.sB, w.rh, w.S, max_rounds);
+                if (e != cudaSuccess) return DCM_E_CUDA;
             }
             post_launch(st);
             if (w.graph && w.emit) return cudaPeekAtLastError() == cudaSuccess ? DCM_OK : DCM_E_CUDA;

@@ -1,0 +1,87 @@
+"""CPU tests of the library's host code where a device call fails: its objects are
+linked against a stand-in for the CUDA runtime (fake/cudart.cpp: two devices,
+kernels recorded by name and not run), which refuses launches or delays events
+as a test asks.  Each test runs in a process of its own."""
+import os
+import shutil
+import subprocess
+import sys
+
+import pytest
+
+from conftest import PKG_DIR, ROOT
+
+FAKE = os.path.join(ROOT, "tests", "fake", "cudart.cpp")
+NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
+
+PRELUDE = """
+import ctypes, os, sys, threading, time
+import numpy as np
+sys.path.insert(0, %r)
+from conftest import load_dcm
+dcm = load_dcm()
+dcm.LIBPATH = sys.argv[1]
+fake = ctypes.CDLL(sys.argv[1])
+cases = __import__("dcm_b200.cases", fromlist=["cases"])
+
+def grid(ip, jp, kp):
+    return cases.make_grid(ip, jp, kp, 50.0, 50.0, 50.0, [-1.0e4, 1.0e5], [300.0, 300.0])
+
+def field(g):
+    return np.zeros((g.kp + 2, g.jp + 2, g.ip + 2), order="F")
+
+def status(call, *args):
+    try:
+        call(*args)
+    except dcm.DCMError as e:
+        return e.status
+    return 0
+""" % os.path.join(ROOT, "tests")
+
+
+@pytest.fixture(scope="module")
+def fake_lib(tmp_path_factory):
+    cxx = shutil.which("g++")
+    if cxx is None or not os.path.exists(NVCC):
+        pytest.skip("no compilers")
+    sys.path.insert(0, PKG_DIR)
+    import build
+    d = tmp_path_factory.mktemp("fake")
+    lib = str(d / "libdcm_fake.so")
+    inc = os.path.join(os.path.dirname(os.path.dirname(NVCC)), "include")
+    subprocess.run([cxx, "-std=c++17", "-O1", "-fPIC", "-I" + inc, "-c", FAKE, "-o",
+                    str(d / "cudart.o")], check=True)
+    subprocess.run([cxx, "-shared", "-o", lib] + build.objects() + [str(d / "cudart.o"),
+                                                                    "-lpthread"], check=True)
+    return lib
+
+
+def run(fake_lib, script, timeout=60):
+    p = subprocess.run([sys.executable, "-c", PRELUDE + script, fake_lib], timeout=timeout,
+                       stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
+    assert p.returncode == 0, p.stdout[-3000:]
+
+
+def test_small_solve_on_a_second_device(fake_lib):
+    """Clusters of 16 blocks are allowed per device: the small FP64 solve's
+    launch is accepted on both."""
+    run(fake_lib, """
+g = grid(16, 1, 16)
+cores = [dcm.DynamicalCore(g, device=d) for d in (0, 1)]
+for d, core in enumerate(cores):
+    assert status(core.bicgstab, field(g), field(g), field(g), 1e-10) == 0
+    assert fake.fake_launches(b"k_bicgstab_point", d) == 1, d
+""")
+
+
+def test_refused_small_solve_is_an_error(fake_lib):
+    run(fake_lib, """
+g = grid(16, 1, 16)
+core = dcm.DynamicalCore(g)
+fake.fake_refuse(b"k_bicgstab_point")
+assert status(core.bicgstab, field(g), field(g), field(g), 1e-10) == dcm.DCM_E_CUDA
+core.set_small_solver(0)
+fake.fake_refuse(b"k_bicg_post")
+core.solver_graphs(False)
+assert status(core.bicgstab, field(g), field(g), field(g), 1e-10, 0, 3) == dcm.DCM_E_CUDA
+""")
