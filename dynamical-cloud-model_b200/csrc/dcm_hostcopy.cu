@@ -236,6 +236,12 @@ void hostcopy_release() {
 }
 
 cudaError_t hostcopy_h2d(void* dst, const void* src, size_t n, cudaStream_t st) {
+    if (n >= MIN_BYTES) {
+        // an error pending here (a refused launch) is the caller's to hear of;
+        // what follows clears errors of its own
+        const cudaError_t before = cudaGetLastError();
+        if (before != cudaSuccess) return before;
+    }
     if (n >= MIN_BYTES && pageable(src)) {
         const cudaError_t e =
             staged((char*)dst, const_cast<char*>((const char*)src), n, false, st);
@@ -245,6 +251,10 @@ cudaError_t hostcopy_h2d(void* dst, const void* src, size_t n, cudaStream_t st) 
 }
 
 cudaError_t hostcopy_d2h(void* dst, const void* src, size_t n, cudaStream_t st) {
+    if (n >= MIN_BYTES) {
+        const cudaError_t before = cudaGetLastError();
+        if (before != cudaSuccess) return before;
+    }
     if (n >= MIN_BYTES && pageable(dst)) {
         const cudaError_t e = staged(const_cast<char*>((const char*)src), (char*)dst, n, true, st);
         if (e != cudaErrorNotReady) return e;

@@ -85,3 +85,19 @@ fake.fake_refuse(b"k_bicg_post")
 core.solver_graphs(False)
 assert status(core.bicgstab, field(g), field(g), field(g), 1e-10, 0, 3) == dcm.DCM_E_CUDA
 """)
+
+
+@pytest.mark.parametrize("kernel", ["k_repitch", "k_unpitch", "k_exchange"])
+@pytest.mark.parametrize("shape", [(16, 12, 10), (64, 64, 64)])
+def test_refused_launch_between_copies_is_an_error(fake_lib, shape, kernel):
+    """A launch refused before or between the copies of a call is that call's
+    error, below and above the size from which threads copy, and not the next
+    call's."""
+    run(fake_lib, """
+g = grid(*%r)
+core = dcm.DynamicalCore(g)
+fake.fake_refuse(%r)
+assert status(core.exchange_along_dim_wo, field(g)) == dcm.DCM_E_CUDA
+fake.fake_refuse(b"")
+assert status(core.exchange_along_dim_wo, field(g)) == 0
+""" % (shape, kernel.encode()))
