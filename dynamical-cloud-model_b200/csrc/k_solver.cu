@@ -91,6 +91,9 @@ struct SolverArgs {
     // mixed form: the iterations follow direct corrections, whose counts and
     // rounds they continue
     int after_direct = 0;
+    // ... from the pressure as corrected: the early return's halo rows, which
+    // belong to an unchanged pressure, are not due
+    int corrected = 0;
     // |omega| below this ends an FP64 solve with DCM_E_BREAKDOWN; the
     // reference's tiny is the default-real literal 1.e-16 (dynamics.f90:321)
     double tiny = (double)1.e-16f;
@@ -2432,7 +2435,7 @@ __global__ void __launch_bounds__(256) k_ru_residual(SolverArgs a, Coef<double> 
         S->cycle_it = 0;
         if (err < a.tol) {
             S->done = 1;
-            S->early = FIRST ? 1 : 0;
+            S->early = FIRST && !a.corrected ? 1 : 0;
         } else if (!(err == err)) {
             S->status = DCM_E_NONFINITE;
             S->done = 1;
@@ -2529,6 +2532,7 @@ int refine_run(SolverWork<float>& wf, SolverWork<double>& wd, const Dims& d, dou
     const bool direct = wf.direct && wf.direct->ok;
     double* const keep = direct && wf.direct->keep ? wf.x_keep : nullptr;
     a.after_direct = direct ? 1 : 0;
+    a.corrected = direct && !keep ? 1 : 0;
     const int max_rounds = wf.round_budget > 0 ? wf.round_budget : itmax + max_updates + 1;
     auto start = [&](cudaStream_t s) { k_ru_begin<<<1, 1, 0, s>>>(wf.S, delta); };
     // the residual of a direct phase; the correction it calls for

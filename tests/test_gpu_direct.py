@@ -9,6 +9,8 @@ handful of corrections, and the fields agree with the FP64 path's within the
 mixed form's bars (1e-6 for p, whose right-hand side FP32 sources perturb;
 1e-5 for the others).
 """
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -170,3 +172,62 @@ def test_pressure_is_put_back_for_the_iterations(dcm):
     start = state.p[1:-1, 1:-1, 1:-1]
     assert np.array_equal(out[0], start)
     assert np.array_equal(out[1], out[2]) and not np.array_equal(out[1], start)
+
+
+def _one_step(dcm, g, state, ptol, graphs=1, max_rounds=0):
+    """(status, statistics, fields) of one mixed step, failed ones too."""
+    core = dcm.DynamicalCore(g)
+    core.solver_graphs(graphs)
+    core.upload_state(state, 1.0, ptol=ptol, kord=3, precision=1)
+    core.driver_start()
+    core.solver_limits(max_rounds=max_rounds)
+    s = dcm.StepStats()
+    status = core.lib.dcm_step(core.h, 1, ctypes.byref(s))
+    f = core.download_state()
+    core.close()
+    return status, s, f
+
+
+def test_iterations_that_follow_a_correction_converge(dcm):
+    """A starting pressure that is the longest wave alone, at rest: the first
+    correction lowers its residual by less than a factor of 4, and the
+    iterations take it below the tolerance (1e-3 of it), from a graph and from
+    the host alike; the residual of the result is the one reported."""
+    ip, jp, kp = 256, 64, 40
+    g = cases.make_grid(ip, jp, kp, 600.0, 600.0, 20.0, [-1.0e4, 1.0e5], [300.0, 300.0])
+    p = cases.fzeros(kp, jp, ip)
+    lam = (2.0 * np.sin(np.pi / ip) / 600.0) ** 2
+    p[1:-1, 1:-1, 1:-1] = np.cos(2 * np.pi * np.arange(ip) / ip + 0.3)[None, None, :] / lam
+    state = cases.State(*(cases.fzeros(kp, jp, ip) for _ in range(10)), p)
+    start = np.sqrt(0.5 * ip * jp * kp) / 0.01  # ||A p|| / 0.01
+    out = []
+    for graphs in (1, 0):
+        status, s, f = _one_step(dcm, g, state, 1e-3 * start, graphs)
+        assert status == 0 and s.err_last < 1e-3 * start
+        assert s.iters_last > 1 and s.iters_last != s.updates_last
+        c = f["p"][1:-1, 1:-1, 1:-1]
+        ax = (np.concatenate([c[1:], c[-1:]]) + np.concatenate([c[:1], c[:-1]]) - 2 * c) / 400.0
+        ax += sum(np.roll(c, q, a) - c for a in (1, 2) for q in (-1, 1)) / 360000.0
+        assert abs(np.sqrt(np.sum(ax ** 2)) / 0.01 - s.err_last) <= 1e-6 * s.err_last
+        out.append((s.iters_last, s.updates_last, f))
+    assert out[0][:2] == out[1][:2]
+    for n in ("u", "v", "w", "p"):
+        assert np.array_equal(out[0][2][n], out[1][2][n]), n
+
+
+def test_iterations_that_follow_corrections_at_round_off(dcm):
+    """A tolerance below what FP64 resolves: corrections until round-off, then
+    the iterations up to itmax; the pressure stays what the corrections reached
+    (the mixed form's bar against the FP64 path's)."""
+    c = cases.warm_bubble(ip=64, jp=64, kp=33, dxyz=50.0, radius=400.0, zc=500.0, seed=66)
+    core = dcm.DynamicalCore(c.grid)
+    core.upload_state(c.state, c.dt, ptol=1e-20, kord=c.kord, precision=1, itmax=9)
+    core.driver_start()
+    s = dcm.StepStats()
+    assert core.lib.dcm_step(core.h, 1, ctypes.byref(s)) == dcm.DCM_E_NOCONV
+    assert s.iters_last >= 9 and 3 <= s.updates_last < s.iters_last
+    m = (slice(1, -1),) * 3
+    p = core.download_state()["p"][m]
+    core.close()
+    q = _steps(dcm, c, 0, nsteps=1)[1]["p"][m]
+    assert relerr(p - p.mean(), q - q.mean()) <= 1e-6
