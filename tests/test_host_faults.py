@@ -101,3 +101,48 @@ assert status(core.exchange_along_dim_wo, field(g)) == dcm.DCM_E_CUDA
 fake.fake_refuse(b"")
 assert status(core.exchange_along_dim_wo, field(g)) == 0
 """ % (shape, kernel.encode()))
+
+
+@pytest.mark.parametrize("mb", [3, 17])
+def test_copies_behind_unfinished_work_cost_no_cores(fake_lib, mb):
+    """A copy that waits for the device sleeps: every DMA here takes 0.2 s, and
+    the process uses less than a fifth of one core meanwhile (the arrays' bytes,
+    and no looking around for longer than a moment, by any thread)."""
+    run(fake_lib, """
+import resource
+def used():
+    r = resource.getrusage(resource.RUSAGE_SELF)
+    return r.ru_utime + r.ru_stime
+g = grid(128, 126, %d)
+core = dcm.DynamicalCore(g)
+a = field(g)
+a[...] = 1.0
+core.exchange_along_dim_wo(a)  # threads, buffers and pages are made
+fake.fake_busy(200)
+t, c = time.time(), used()
+core.exchange_along_dim_wo(a)
+t, c = time.time() - t, used() - c
+assert t >= 0.4, t
+assert c <= 0.2 * t, (c, t)
+""" % (mb * 1000000 // (8 * 130 * 128)))
+
+
+def test_copies_move_every_byte(fake_lib):
+    """Arrays of every number of buffers, through threads that sleep and wake
+    between the chunks (each DMA takes longer than a thread looks for work) and
+    that do not.  The kernels between do nothing: an upload's bytes stay in the
+    stage, from where the download returns them."""
+    run(fake_lib, """
+rng = np.random.default_rng(5)
+for kp in (62, 14, 30, 61, 93, 130):
+    g = grid(128, 252, kp)
+    core = dcm.DynamicalCore(g)
+    for ms in (0, 2, 0):
+        fake.fake_busy(ms)
+        a = field(g)
+        a[...] = rng.normal(size=a.shape)
+        want = a.copy(order="F")
+        core.exchange_along_dim_wo(a)
+        assert np.array_equal(a, want)
+    core.close()
+""")
