@@ -3,6 +3,7 @@
 
 #include <emmintrin.h>
 #include <sched.h>
+#include <unistd.h>
 
 #include <algorithm>
 #include <atomic>
@@ -93,6 +94,8 @@ void stream_copy(char* dst, const char* src, size_t n) {
 // they have woken (up to a millisecond on an idle host).
 class Copier {
 public:
+    // false in a child process, which has the object but none of its threads
+    bool here() const { return owner_ == getpid(); }
     // false when the page-locked buffers cannot be had
     bool start() {
         if (started_) return true;
@@ -261,6 +264,7 @@ private:
     std::vector<std::thread> threads_;
     std::mutex m_;
     std::condition_variable cv_;
+    const pid_t owner_ = getpid();
     bool started_ = false, quit_ = false, down_ = false;
     unsigned long job_ = 0;
     char* host_ = nullptr;
@@ -298,6 +302,10 @@ void hostcopy_retain() {
 void hostcopy_release() {
     std::lock_guard<std::mutex> l(g_count_lock);
     if (--g_handles > 0) return;
+    if (g_copier && !g_copier->here()) {  // left as it is: there are no threads to join
+        g_copier = nullptr;
+        return;
+    }
     std::lock_guard<std::mutex> c(g_copier_lock);
     delete g_copier;
     g_copier = nullptr;

@@ -146,3 +146,30 @@ for kp in (62, 14, 30, 61, 93, 130):
         assert np.array_equal(a, want)
     core.close()
 """)
+
+
+def test_forked_child_gives_up_its_handle(fake_lib):
+    """A child process has the handle but not the threads that copy: it can
+    destroy the handle (the binding does when the object goes) and exit."""
+    run(fake_lib, """
+g = grid(64, 64, 64)
+core = dcm.DynamicalCore(g)
+assert status(core.exchange_along_dim_wo, field(g)) == 0
+pid = os.fork()
+if pid == 0:
+    core.close()
+    os._exit(7)
+end = time.time() + 20
+while time.time() < end:
+    done, st = os.waitpid(pid, os.WNOHANG)
+    if done:
+        break
+    time.sleep(0.05)
+else:
+    os.kill(pid, 9)
+    os.waitpid(pid, 0)
+    raise AssertionError("the child hangs")
+assert os.WEXITSTATUS(st) == 7
+assert status(core.exchange_along_dim_wo, field(g)) == 0
+core.close()
+""")
