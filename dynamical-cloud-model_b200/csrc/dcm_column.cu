@@ -458,32 +458,49 @@ extern "C" int dcm_mpdata_vec_1d_device(int ncol, int kp, int nq, int l_h, int r
 }
 
 // Device memory of the host-array calls, kept by the thread that makes them
-// (at most 32 MB, on one device) and freed when it ends: a cudaMalloc and the
+// (at most 32 MB, of one context) and freed when it ends: a cudaMalloc and the
 // cudaFree, which waits for the device, took most of a call of a few hundred
 // columns.  A thread's calls return after their last copy, so its next call
-// finds the memory free.
+// finds the memory free.  It is used in, and given back to, the context it
+// came from only: contexts are told apart by the driver's identifiers, which
+// are not used twice.
 namespace {
 constexpr size_t COL_KEEP = 32u << 20;
 constexpr size_t COL_PACK = 16u << 10;  // small arrays that go in one copy
+
+// the current context's identifier, 0 where there is none yet (or no way to ask)
+unsigned long long context_id() {
+    using Ask = int (*)(void*, unsigned long long*);  // cuCtxGetId
+    static const Ask ask = [] {
+        void* f = nullptr;
+        cudaDriverEntryPointQueryResult found;
+        if (cudaGetDriverEntryPoint("cuCtxGetId", &f, cudaEnableDefault, &found) != cudaSuccess)
+            cudaGetLastError();
+        else if (found == cudaDriverEntryPointSuccess)
+            return (Ask)f;
+        return (Ask) nullptr;
+    }();
+    unsigned long long id = 0;
+    return ask && ask(nullptr, &id) == 0 ? id : 0;
+}
+
 struct ColSpace {
     char* p = nullptr;
     size_t n = 0;
-    int device = -1;
+    unsigned long long context = 0;
+    // (memory of another context is left to that context's end)
     void drop() {
-        int now = 0;
-        if (p && cudaGetDevice(&now) == cudaSuccess && cudaSetDevice(device) == cudaSuccess) {
-            cudaFree(p);
-            cudaSetDevice(now);
-        }
+        if (p && context_id() == context) cudaFree(p);
         p = nullptr;
         n = 0;
     }
     bool take(size_t want, char** out) {
-        int now = 0;
-        if (want > COL_KEEP || cudaGetDevice(&now) != cudaSuccess) return false;
-        if (want > n || now != device) {
+        if (want > COL_KEEP) return false;
+        const unsigned long long now = context_id();
+        if (now == 0) return false;
+        if (want > n || now != context) {
             drop();
-            device = now;
+            context = now;
             const size_t size = std::min(COL_KEEP, want + want / 2);
             if (cudaMalloc(&p, size) != cudaSuccess) {
                 cudaGetLastError();

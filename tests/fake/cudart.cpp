@@ -6,6 +6,7 @@
 // Refusals and delays, set by the tests:
 //   fake_refuse(text)    launches of kernels whose name contains text fail
 //   fake_busy(ms)        an event is done that long after its record
+//   fake_context(id)     the current context; memory of another one is refused
 //   fake_launches(text, device)  accepted launches so far (device < 0: all)
 #include <cuda_runtime_api.h>
 
@@ -27,6 +28,11 @@ struct Launch {
     std::string name;
     int device;
 };
+struct Block {
+    size_t n;
+    bool host;
+    unsigned long long context;
+};
 struct Event {
     Clock::time_point done{};
 };
@@ -43,7 +49,8 @@ std::map<const void*, std::string>& kernels() {
     return m;
 }
 std::map<std::pair<int, const void*>, bool> large;     // non-portable clusters allowed
-std::map<const char*, std::pair<size_t, bool>> blocks;  // address -> size, on the host
+std::map<const char*, Block> blocks;  // by address
+unsigned long long context = 1;
 std::vector<Launch> launches;
 std::string refuse;
 int busy_ms = 0;
@@ -67,7 +74,7 @@ cudaError_t launch(const void* f, unsigned cluster) {
 cudaError_t take(void** p, size_t n, bool host) {
     *p = std::calloc(n ? n : 1, 1);
     std::lock_guard<std::mutex> l(mu);
-    blocks[(const char*)*p] = {n, host};
+    blocks[(const char*)*p] = {n, host, context};
     return cudaSuccess;
 }
 cudaError_t give(void* p) {
@@ -78,6 +85,23 @@ cudaError_t give(void* p) {
     }
     std::free(p);
     return cudaSuccess;
+}
+cudaError_t copy(void* d, const void* s, size_t n) {
+    {
+        std::lock_guard<std::mutex> l(mu);
+        for (const char* p : {(const char*)d, (const char*)s}) {
+            auto it = blocks.upper_bound(p);
+            if (it == blocks.begin() || p >= (--it)->first + it->second.n) continue;
+            if (!it->second.host && it->second.context != context)
+                return set(cudaErrorInvalidValue);
+        }
+    }
+    std::memcpy(d, s, n);
+    return cudaSuccess;
+}
+int context_id(void*, unsigned long long* id) {
+    *id = context;
+    return 0;
 }
 unsigned cluster_of(const cudaLaunchConfig_t* c) {
     for (unsigned q = 0; q < c->numAttrs; q++)
@@ -94,6 +118,10 @@ extern "C" {
 void fake_refuse(const char* text) {
     std::lock_guard<std::mutex> l(mu);
     refuse = text;
+}
+void fake_context(unsigned long long id) {
+    std::lock_guard<std::mutex> l(mu);
+    context = id;
 }
 void fake_busy(int ms) { busy_ms = ms; }
 int fake_launches(const char* text, int device) {
@@ -181,16 +209,19 @@ cudaError_t cudaPointerGetAttributes(cudaPointerAttributes* a, const void* p) {
     a->type = cudaMemoryTypeUnregistered;
     std::lock_guard<std::mutex> l(mu);
     auto it = blocks.upper_bound((const char*)p);
-    if (it != blocks.begin() && (const char*)p < (--it)->first + it->second.first)
-        a->type = it->second.second ? cudaMemoryTypeHost : cudaMemoryTypeDevice;
+    if (it != blocks.begin() && (const char*)p < (--it)->first + it->second.n)
+        a->type = it->second.host ? cudaMemoryTypeHost : cudaMemoryTypeDevice;
     return cudaSuccess;
 }
-cudaError_t cudaMemcpy(void* d, const void* s, size_t n, cudaMemcpyKind) {
-    std::memcpy(d, s, n);
-    return cudaSuccess;
-}
+cudaError_t cudaMemcpy(void* d, const void* s, size_t n, cudaMemcpyKind) { return copy(d, s, n); }
 cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, cudaMemcpyKind, cudaStream_t) {
-    std::memcpy(d, s, n);
+    return copy(d, s, n);
+}
+cudaError_t cudaGetDriverEntryPoint(const char* name, void** f, unsigned long long,
+                                    cudaDriverEntryPointQueryResult* r) {
+    const bool known = !std::strcmp(name, "cuCtxGetId");
+    *f = known ? (void*)context_id : nullptr;
+    if (r) *r = known ? cudaDriverEntryPointSuccess : cudaDriverEntryPointSymbolNotFound;
     return cudaSuccess;
 }
 cudaError_t cudaMemset(void* d, int v, size_t n) {

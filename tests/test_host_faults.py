@@ -173,3 +173,19 @@ assert os.WEXITSTATUS(st) == 7
 assert status(core.exchange_along_dim_wo, field(g)) == 0
 core.close()
 """)
+
+
+def test_column_memory_stays_with_its_context(fake_lib):
+    """The device memory that a thread keeps for the sedimentation calls is used
+    again in the context that it came from, and not in another on the same
+    device."""
+    run(fake_lib, """
+ncol, kp = 7, 20
+met = [np.ones(kp + 2) for _ in range(4)]
+w, psi = np.zeros((ncol, kp + 2)), np.ones((ncol, 1, kp + 2))
+def call():
+    return status(lambda: dcm.mpdata_vec_1d_columns(1.0, 1, *met, w, psi))
+for c in (1, 1, 2, 2, 1):
+    fake.fake_context(ctypes.c_ulonglong(c))
+    assert call() == 0, c
+""")
