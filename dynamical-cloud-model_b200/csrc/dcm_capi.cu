@@ -112,7 +112,7 @@ struct dcm_handle {
     // dcm_set_small_solver: FP64 solves of at most this many interior points
     // run as one thread-block cluster
     long long small_max = 8192;
-    int small_blocks = 8;  // of this handle's device
+    int small_most = 8, small_blocks = 8;  // blocks the device can place, blocks taken
     // dcm_set_mpdata_shape: fused antidiffusive iterations (off by default:
     // slower on B200, see dcm.h), their row cap
     int mp_fuse = 0, mp_rows = 32;
@@ -404,7 +404,7 @@ extern "C" int dcm_create(const dcm_grid* g, int device, dcm_handle** out) {
     h->nh = h->hd.n();
     CK(cudaSetDevice(device));
     CK(cudaStreamCreateWithFlags(&h->st, cudaStreamNonBlocking));
-    h->small_blocks = solver_init();
+    h->small_most = h->small_blocks = solver_init();
     mpdata_init();
     direct_init();
     CK(cudaEventCreate(&h->ev0));
@@ -1535,6 +1535,17 @@ extern "C" int dcm_set_small_solver(dcm_handle* h, int max_points) {
     if (max_points < 0) return fail(h, DCM_E_ARG, "set_small_solver: max_points");
     if (max_points != h->small_max) h->generation += 1;
     h->small_max = max_points;
+    return DCM_OK;
+}
+
+extern "C" int dcm_set_small_cluster(dcm_handle* h, int blocks) {
+    CHECK_H();
+    if (blocks != 0 && blocks != 8 && blocks != 16)
+        return fail(h, DCM_E_ARG, "set_small_cluster: blocks");
+    if (blocks > h->small_most) return fail(h, DCM_E_UNSUPPORTED, "set_small_cluster: blocks");
+    const int b = blocks ? blocks : h->small_most;
+    if (b != h->small_blocks) h->generation += 1;
+    h->small_blocks = b;
     return DCM_OK;
 }
 

@@ -387,6 +387,11 @@ int dcm_solver_graphs(dcm_handle *h, int on);
  * statuses and the iteration counts reported are those of the multi-kernel
  * solve. */
 int dcm_set_small_solver(dcm_handle *h, int max_points);
+/* The blocks of that cluster for domains of at most 8192 points: 16 (of 512
+ * threads; DCM_E_UNSUPPORTED where the device cannot place such a cluster), 8
+ * (of 1024), or 0, the default: 16 where it can be placed.  Both form the same
+ * sums in the same order: the results are bit-identical. */
+int dcm_set_small_cluster(dcm_handle *h, int blocks);
 
 /* MPDATA launch shape (no counterpart in the reference).  fuse = 0 (the
  * default): one kernel per stage of an antidiffusive iteration

@@ -71,6 +71,8 @@ cores = [dcm.DynamicalCore(g, device=d) for d in (0, 1)]
 for d, core in enumerate(cores):
     assert status(core.bicgstab, field(g), field(g), field(g), 1e-10) == 0
     assert fake.fake_launches(b"k_bicgstab_point", d) == 1, d
+assert status(cores[1].set_small_cluster, 8) == 0
+assert status(cores[1].set_small_cluster, 12) == dcm.DCM_E_ARG
 """)
 
 
