@@ -231,3 +231,37 @@ def test_iterations_that_follow_corrections_at_round_off(dcm):
     core.close()
     q = _steps(dcm, c, 0, nsteps=1)[1]["p"][m]
     assert relerr(p - p.mean(), q - q.mean()) <= 1e-6
+
+
+def test_corrections_in_an_ensemble(dcm):
+    """Members whose solves take direct corrections (one on flat cells, whose
+    pressure is kept) beside one that iterates: the captured steps give the
+    members' own, also over an upload that keeps them."""
+    cs = [(c.grid, c.state, c.kord) for c in (
+        cases.warm_bubble(ip=64, jp=64, kp=33, dxyz=50.0, radius=400.0, zc=500.0, seed=66),
+        cases.warm_bubble(ip=24, jp=20, kp=16, dxyz=100.0, radius=500.0, zc=800.0, seed=67),
+        cases.warm_bubble(ip=72, jp=50, kp=41, dxyz=50.0, radius=400.0, zc=500.0, seed=68))]
+    cs.append(_flat((64, 64, 40), 4000.0, 4000.0, 20.0) + (3,))
+    ens = dcm.Ensemble([c[0] for c in cs])
+
+    def start(core, c):
+        core.upload_state(c[1], 1.0, ptol=1e-10, kord=c[2], precision=1)
+        core.driver_start()
+    alone = []
+    for c in cs:
+        core = dcm.DynamicalCore(c[0])
+        start(core, c)
+        for _ in range(4):
+            s = core.step(1)
+        alone.append((s.iters_last, core.download_state()))
+        core.close()
+    assert [a[0] > 5 for a in alone] == [False, True, False, False]
+    for _ in range(2):
+        for core, c in zip(ens.members, cs):
+            start(core, c)
+        ens.step(4)
+        for core, (_, f) in zip(ens.members, alone):
+            g = core.download_state()
+            for n in ("u", "v", "w", "th", "p"):
+                assert np.array_equal(g[n], f[n]), n
+    ens.close()
