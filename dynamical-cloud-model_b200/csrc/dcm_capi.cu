@@ -1060,7 +1060,7 @@ SolverWork<float> solver_work_f(dcm_handle* h) {
     w.round_budget = h->round_budget;
     w.direct = &h->direct;
     if (h->direct.keep) {  // the pressure at the start; without it the iterations alone
-        w.x_keep = slot(h, S_X);
+        w.x_keep = slot(h, S_STAGE);  // between downloads, which also use it
         if (!w.x_keep) {
             cudaGetLastError();
             w.direct = nullptr;
@@ -1462,6 +1462,9 @@ extern "C" int dcm_state_upload(dcm_handle* h, const dcm_config* cfg, const dcm_
     h->q2.assign(nqq, 0.0);
     h->t1 = h->t2 = 0.0;  // saved locals, :260
     h->refine_outer_total = 0;
+    // the kept pressure of solver_work_f, zeroed before a step writes it (an
+    // ensemble's step runs on other streams)
+    if (h->prec == 1 && h->direct.keep && !slot(h, S_STAGE)) cudaGetLastError();
     h->resident = true;
     return sync(h);
 }
