@@ -9,7 +9,9 @@
 // and the limiter's beta_up / beta_down sit in shared memory; every statement
 // of the Fortran is a pass of the 32 lanes over the levels, separated by
 // __syncwarp.  Reductions over k (minval, the positivity test's sum) are warp
-// shuffles.  All arithmetic is FP64 in the reference's order of terms.
+// shuffles.  All arithmetic is FP64, in the reference's order of terms but for
+// k_column_donor, which forms one reciprocal per level and rounds otherwise (up
+// to 4e-16 of a column's largest value).
 #include <algorithm>
 #include <cstring>
 

@@ -46,10 +46,10 @@ struct Coef {
 // ---- direct corrections of the mixed form's solve (k_direct.cu) -------------
 // The domains that take them, by interior points.  Measured per step (mixed
 // form, precond 1, iterations -> corrections): 97x75x61 7.4 -> 0.4 ms,
-// 256x256x128 34 -> 2.0 ms.  Smaller domains would gain too, but keep the
-// FP32 iterations: a step of 81x45x32 takes 4 ms, and the iteration counts
-// that dcm_step reports there are what the sweeps and launch shapes are
-// compared by.  Larger ones keep them because of p's additive constant, which
+// 256x256x128 34 -> 2.0 ms.  Smaller domains would gain too (a step of 81x45x32
+// takes 4 ms), but keep the FP32 iterations: the line lies above the domains
+// whose reported iteration counts the sweeps and launch shapes are compared
+// by, up to 48x48x32.  Larger ones keep them because of p's additive constant, which
 // no velocity depends on: there the iterations' round-off and restarts move
 // it (2 of 21 seeded 384x256x256 convections: a mean of 4 % of p's spread,
 // and far above it), so a corrected solve would return another p.  Up to

@@ -279,7 +279,7 @@ __device__ __forceinline__ void fft_pass_of(int radix, int n, int ns,
 // exchanged.  256 x 256 x 128: 27 us a transform (67 MB, 10 us at the copy rate;
 // half of the field comes from L2), bound by instruction fetch (the unrolled
 // radices, a third of the stalls) and by loads in flight at 80 registers;
-// FFT_ADD 66 us (168 MB, 26 us), bound by the wait for x.
+// FFT_ADD 44 us (168 MB, 26 us), bound by the wait for x.
 enum FftMode {
     FFT_REAL = 0,  // forward, of a real field
     FFT_FWD,       // forward, of complex pairs
