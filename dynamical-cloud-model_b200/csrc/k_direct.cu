@@ -783,8 +783,9 @@ __global__ void __launch_bounds__(256, 4) k_dir_residual(DirResidualArgs a, Red2
     } else if (FIRST && !(err == err)) {
         S->status = DCM_E_NONFINITE;
         S->done = 1;
-    } else if (FIRST || err <= DIRECT_CONTRACTION * S->err) {
-        // another correction, within the limits of the iterations
+    } else if (FIRST || err < DIRECT_CONTRACTION * S->err) {
+        // another correction, within the limits of the iterations (none from
+        // an infinite residual to an infinite one)
         if (S->it >= a.itmax) {
             S->status = DCM_E_NOCONV;
             S->done = 1;

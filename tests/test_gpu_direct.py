@@ -265,3 +265,16 @@ def test_corrections_in_an_ensemble(dcm):
             for n in ("u", "v", "w", "th", "p"):
                 assert np.array_equal(g[n], f[n]), n
     ens.close()
+
+
+@pytest.mark.parametrize("graphs", [1, 0])
+@pytest.mark.parametrize("value,size", [(np.inf, None), (1e200, 1e200)])
+def test_corrections_end_at_an_infinite_residual(dcm, value, size, graphs):
+    """A residual whose norm overflows contracts under no correction: after one
+    the iterations take over, which end the step as they do without it."""
+    c = cases.warm_bubble(ip=64, jp=64, kp=33, dxyz=50.0, radius=400.0, zc=500.0, seed=66)
+    if size:
+        c.state.p[1:-1, 1:-1, 1:-1] = size * np.random.default_rng(69).normal(size=(33, 64, 64))
+    c.state.p[5, 6, 7] = value
+    status, s, _ = _one_step(dcm, c.grid, c.state, 1e-10, graphs)
+    assert status == dcm.DCM_E_NOCONV and s.iters_last <= 1 and np.isinf(s.err_last)
